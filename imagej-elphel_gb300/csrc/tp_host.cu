@@ -171,6 +171,19 @@ static size_t strips_need(const tp_handle *h) {
   return (size_t)h->ntiles * (h->num_pairs > 0 ? h->num_pairs : 1) * RE;
 }
 
+// the pair list of tp_quad_pairs (Correlation2d.PAIRS): the forward then takes the six pairs together
+static int is_standard_quad(const tp_handle *h) {
+  tp_pair q[6];
+  int n = 0;
+  tp_quad_pairs(q, &n);
+  if (h->cfg.num_sensors != 4 || h->num_pairs != n || h->corr_host.log_combine) return 0;
+  for (int i = 0; i < n; i++) {
+    const PairDev &p = h->corr_host.pairs[i];
+    if (p.cam1 != q[i].cam1 || p.cam2 != q[i].cam2 || p.kind != q[i].kind) return 0;
+  }
+  return 1;
+}
+
 static SceneDev scene_of(tp_handle *h) {
   SceneDev sc;
   memset(&sc, 0, sizeof(sc));
@@ -221,6 +234,7 @@ static SceneDev scene_of(tp_handle *h) {
   sc.num_pairs = h->num_pairs;
   sc.strip_rows = h->corr_host.strip_rows;
   sc.wndy_size = h->corr_host.wndy_size;
+  sc.quad_std = is_standard_quad(h);
   return sc;
 }
 
@@ -433,6 +447,7 @@ tp_status tp_create(const tp_config *cfg, tp_handle **out) {
   ok = ok && cudaEventCreateWithFlags(&h->ev_work, cudaEventDisableTiming) == cudaSuccess;
   ok = ok && upload_kernel_constants() == cudaSuccess;
   ok = ok && upload_fused_constants() == cudaSuccess;
+  ok = ok && upload_quad_constants() == cudaSuccess;
   ok = ok && upload_texture_constants() == cudaSuccess;
   ok = ok && upload_adjoint_constants() == cudaSuccess;
   ok = ok && upload_kernprep_constants() == cudaSuccess;

@@ -15,6 +15,7 @@
 #define TP_MAXP 120
 #define TP_MAX_STRIP 16     // rows of the combined strip
 #define TP_NDISP 9
+#define TP_BATCH_MAX 256      // scenes of a batch
 
 // one (task, sensor, colour) sub-tile: integer window corner, residual shift
 // and kernel-table index, computed in FP64 by the plan kernel
@@ -123,6 +124,7 @@ struct SceneDev {
   int num_pairs;             // host copy of corr_cfg->num_pairs (launch sizing)
   int strip_rows;            // host copy of corr_cfg->strip_rows
   int wndy_size;             // host copy of corr_cfg->wndy_size
+  int quad_std;              // the pairs are the six of a standard quad, in its order (is_standard_quad)
 };
 
 // texture-tile settings (CLTParameters defaults in tp_host.cu), read uniformly
@@ -155,6 +157,15 @@ cudaError_t upload_kernel_constants();
 // tpb/nw = tiles and warps per CTA (<= 0: defaults for the sensor/colour layout)
 cudaError_t launch_fused_forward(const SceneDev &sc, const CorrConst &cc, int tpb, int nw, cudaStream_t st);
 cudaError_t upload_fused_constants();
+// standard quads (tp_quad.cu): whether a scene (a batch's scenes) takes that path, and its launches
+cudaError_t upload_quad_constants();
+bool quad_forward_ok(const SceneDev &sc);
+cudaError_t launch_quad_forward(const SceneDev &sc, const CorrConst &cc, int nw, cudaStream_t st);
+bool quad_batch_ok(const SceneDev *scenes_host, int n);
+cudaError_t launch_quad_batch(const SceneDev *scenes_host, const SceneDev *scenes_dev, const int *unit_off_dev, int n,
+                              int total_units, cudaStream_t st);
+// phase C of a forward that left its strip and ortho profile products in sc.combo and sc.osum
+cudaError_t launch_extract_pass(const SceneDev &sc, const CorrConst &cc, int quad, int RE, cudaStream_t st);
 // GPU_DTT24_DRV counterpart (tp_fused.cu): 2D DTT of one mode on every 8x8 block
 cudaError_t launch_dtt8x8(float *dst, const float *src, int stride, int width, int height, int mode,
                           cudaStream_t st);

@@ -1,0 +1,328 @@
+// tp_quad.cu -- the forward of standard quads (4 sensors, the six pairs of Correlation2d.PAIRS, mono or
+// Bayer, all images of one type): the shape of nearly every scene, so it has its own kernels.
+//
+// A warp carries a tile through all stages, as in the general warp-per-tile schedule, with three
+// differences: the image windows are staged in shared memory one item ahead (tp_forward.cuh), the
+// six pairs are taken together two values per instruction (tp_pairs.cuh), and the extraction's serial
+// half runs as a pass of its own (extract_kernel).
+//
+// Measured (kernel and extraction together, before -> now): 4x2592x1936 u16 Bayer with kernel tables,
+// 78,408 tiles: 0.922 -> 0.813 ms; 4x1304x984 float Bayer, 7,018 tiles: 129 -> 82 us; 16 batched
+// 4x512x384 float mono scenes, 49,152 tiles: 452 -> 334 us.  What bounds it now: latency at 16 warps
+// an SM (128 registers a thread): the issue slots are about half used, the shared-memory pipe
+// 60 % (Bayer) to 68 % (mono).
+//
+// Shared memory of a warp (floats): CLT [C][4 sensors][256] first; the windows of colour item c at
+// 1024 c (where that item's CLT goes once they are read); the pairs' spectra over the CLT
+// (QP_SURF floats), then the surfaces; transpose buffers behind the CLT.
+#include "tp_forward.cuh"
+#include "tp_pairs.cuh"
+#include "tp_launch.h"
+
+namespace {
+
+__host__ __device__ constexpr int quad_warp_floats(int C) { return C == 3 ? 3 * 1024 + SCR : QP_FLOATS; }
+__host__ __device__ constexpr int quad_tbuf(int C) { return C == 3 ? 3 * 1024 : 1300; }
+
+__device__ __forceinline__ SubtilePlan quad_plan(const SceneDev &sc, int C, int task, int s, int c) {
+  return sc.plan[((size_t)task * 4 + s) * C + c];
+}
+
+// lane q * 8 + r copies its share of sensor q's window of colour item c
+template <bool U16>
+__device__ __forceinline__ void quad_stage(const SceneDev &sc, const SubtilePlan &p, int c, float *ws, int q, int r) {
+  stage_window<U16>(sc, sc.images[q], p.tlx, p.tly, ws + c * 1024 + q * Stage<U16>::WIN, r);
+  cp_async_commit();
+}
+
+// phase A of a tile: p is the plan of (sensor q, colour 0), whose windows are staged
+template <int C, bool U16>
+__device__ __forceinline__ void quad_clt(const SceneDev &sc, int task, size_t tile, SubtilePlan p, float *ws, int lane) {
+  const int q = lane >> 3, r = lane & 7;
+  const int rr = sc.bayer_red_row, rc = sc.bayer_red_col;
+  float *tbuf = ws + quad_tbuf(C) + q * 72;
+#pragma unroll 1
+  for (int c = 0; c < C; c++) {
+    const SubtilePlan pn = (c + 1 < C) ? quad_plan(sc, C, task, q, c + 1) : p;
+    SWin<U16> w;
+    w.base = (const typename Stage<U16>::T *)(ws + c * 1024 + q * Stage<U16>::WIN);
+    w.sx = p.tlx & (Stage<U16>::CH - 1);
+    w.scale = sc.color_scale[c];
+    cp_async_wait_all();  // this item's windows, copied by every lane
+    __syncwarp();
+    float o[4][8];
+    if (C == 1) {
+      subtile_clt<0>(w, p.rx, p.ry, 0, 0, 0, r, tbuf, o);
+    } else if (c < 2) {
+      const int pc = ((c == 0 ? rc : 1 - rc) - p.tlx) & 1, pr = ((c == 0 ? rr : 1 - rr) - p.tly) & 1;
+      subtile_clt<1>(w, p.rx, p.ry, pc, pr, 0, r, tbuf, o);
+    } else {
+      const int pg = (p.tlx + p.tly + rc + rr + 1) & 1;
+      subtile_clt<2>(w, p.rx, p.ry, 0, 0, pg, r, tbuf, o);
+    }
+    // every lane has read this item's windows (the transposes in subtile_clt synchronise the warp)
+    if (c + 1 < C) quad_stage<U16>(sc, pn, c + 1, ws, q, r);
+    const float *kp = (p.kidx >= 0) ? sc.kernels[q] + (size_t)p.kidx * TP_CLT : nullptr;
+    conv_shift(o, kp, p.rx, p.ry, r);
+    float *sdst = ws + (c * 4 + q) * TP_CLT + r * 8;
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      *(float4 *)(sdst + m * 64) = make_float4(o[m][0], o[m][1], o[m][2], o[m][3]);
+      *(float4 *)(sdst + m * 64 + 4) = make_float4(o[m][4], o[m][5], o[m][6], o[m][7]);
+    }
+    store_clt(sc, c, r, sc.clt + ((tile * 4 + q) * C + c) * TP_CLT + r * 8, o);
+    p = pn;
+  }
+  __syncwarp();
+}
+
+// the products the extraction pass starts from
+template <int NT>
+__device__ __forceinline__ void store_products(const SceneDev &sc, size_t tile, int RE, int lane, const float cmb[8],
+                                               const float oprod[8]) {
+#pragma unroll
+  for (int t = 0; t < NT; t++) {
+    const int e = lane + 32 * t;
+    if (e < RE) sc.combo[tile * RE + e] = cmb[t];
+  }
+  float4 *ob = (float4 *)(sc.osum + (tile * 32 + lane) * 8);
+  ob[0] = make_float4(oprod[0], oprod[1], oprod[2], oprod[3]);
+  ob[1] = make_float4(oprod[4], oprod[5], oprod[6], oprod[7]);
+}
+
+__device__ __forceinline__ size_t tile_of(const SceneDev &sc, int task) {
+  const int txy = sc.task_txy[task];
+  return (size_t)(txy >> 16) * sc.tilesX + (txy & 0xffff);
+}
+
+}  // namespace
+
+template <int C, bool U16, int NT>
+__global__ void __launch_bounds__(128, 4) quad_kernel(const __grid_constant__ SceneDev sc,
+                                                      const __grid_constant__ CorrConst cfg, int RE) {
+  extern __shared__ float sm[];
+  __shared__ float s_lpf[64];  // the correlation LPF, read per lane
+  for (int i = threadIdx.x; i < 64; i += blockDim.x) s_lpf[i] = cfg.lpf[i];
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane >> 3, r = lane & 7, NW = blockDim.x >> 5;
+  float *ws = sm + warp * quad_warp_floats(C);
+  const short *strip_code = &sc.corr_cfg->strip_code[0][0][0];
+  const int stride = gridDim.x * NW;
+  int task = blockIdx.x * NW + warp;
+  SubtilePlan p;
+  size_t tile = 0;
+  if (task < sc.num_tasks) {
+    p = quad_plan(sc, C, task, q, 0);
+    tile = tile_of(sc, task);
+    quad_stage<U16>(sc, p, 0, ws, q, r);
+  }
+  for (; task < sc.num_tasks; task += stride) {
+    quad_clt<C, U16>(sc, task, tile, p, ws, lane);
+    const size_t cur = tile;
+    const int next = task + stride;
+    if (next < sc.num_tasks) {
+      p = quad_plan(sc, C, next, q, 0);
+      tile = tile_of(sc, next);
+    }
+    const float *surf = quad_surfaces<C>(sc, cfg, s_lpf, cur, ws, lane);
+    if (next < sc.num_tasks) quad_stage<U16>(sc, p, 0, ws, q, r);  // the next tile's first windows
+    float cmb[8], oprod[8];
+    quad_strips<NT>(sc, cfg, surf, cur, RE, strip_code, lane, cmb, oprod);
+    store_products<NT>(sc, cur, RE, lane, cmb, oprod);
+    if (C > 1) {  // the next tile's windows and CLT go over the surfaces
+      if (lane == 0) bulk_read_done();
+      __syncwarp();
+    }
+  }
+  cp_async_wait_all();
+  if (lane == 0) bulk_done();
+}
+
+// The same over many mono scenes, a unit of four tiles (of one scene) per CTA and step, as
+// fused_batch_kernel.
+template <bool U16, int NT>
+__global__ void __launch_bounds__(128, 4)
+    quad_batch_kernel(const SceneDev *__restrict__ scenes, const int *__restrict__ unit_off, int nscenes,
+                      int total_units, int cfg_floats) {
+  extern __shared__ float smem[];
+  __shared__ int s_off[TP_BATCH_MAX + 1];
+  __shared__ SceneDev s_sc;
+  CorrConst *s_cfg = (CorrConst *)smem;  // header and the six pairs of the current scene
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane >> 3, r = lane & 7;
+  float *ws = smem + cfg_floats + warp * quad_warp_floats(1);
+  for (int i = threadIdx.x; i <= nscenes; i += blockDim.x) s_off[i] = unit_off[i];
+  int cur = -1;
+  bool staged = false;
+  SubtilePlan p;
+  __syncthreads();
+  for (int u = blockIdx.x; u < total_units; u += gridDim.x) {
+    int lo = 0, hi = nscenes - 1;  // last scene whose first unit is <= u
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (s_off[mid] <= u) lo = mid;
+      else hi = mid - 1;
+    }
+    if (lo != cur) {
+      __syncthreads();
+      const int *src = (const int *)(scenes + lo);
+      for (int i = threadIdx.x; i < (int)(sizeof(SceneDev) / sizeof(int)); i += blockDim.x) ((int *)&s_sc)[i] = src[i];
+      const int cfg_words = (int)((offsetof(CorrConst, pairs) + 6 * sizeof(PairDev)) / sizeof(int));
+      const int *csrc = (const int *)scenes[lo].corr_cfg;
+      for (int i = threadIdx.x; i < cfg_words; i += blockDim.x) ((int *)s_cfg)[i] = csrc[i];
+      cur = lo;
+      __syncthreads();
+    }
+    const SceneDev &sc = s_sc;
+    const CorrConst &cfg = *s_cfg;
+    const int RE = (sc.strip_rows < sc.wndy_size ? sc.strip_rows : sc.wndy_size) * 15;
+    const int task = (u - s_off[lo]) * 4 + warp;
+    const int nu = u + gridDim.x, next = (nu < s_off[lo + 1]) ? (nu - s_off[lo]) * 4 + warp : sc.num_tasks;
+    if (task < sc.num_tasks) {
+      if (!staged) {
+        p = quad_plan(sc, 1, task, q, 0);
+        quad_stage<U16>(sc, p, 0, ws, q, r);
+      }
+      const size_t tile = tile_of(sc, task);
+      quad_clt<1, U16>(sc, task, tile, p, ws, lane);
+      staged = next < sc.num_tasks;  // the next unit's windows, where it is of the same scene
+      if (staged) p = quad_plan(sc, 1, next, q, 0);
+      const float *surf = quad_surfaces<1>(sc, cfg, cfg.lpf, tile, ws, lane);
+      if (staged) quad_stage<U16>(sc, p, 0, ws, q, r);
+      float cmb[8], oprod[8];
+      quad_strips<NT>(sc, cfg, surf, tile, RE, &sc.corr_cfg->strip_code[0][0][0], lane, cmb, oprod);
+      store_products<NT>(sc, tile, RE, lane, cmb, oprod);
+    }
+  }
+  cp_async_wait_all();
+  if (lane == 0) bulk_done();
+}
+
+// Phase C for the tiles of a fused forward that left it out: warp per task, from the strip
+// products (in sc.combo, replaced by the combined strip) and the ortho profile products (sc.osum)
+// the forward wrote.  Phase C is short chains of dependent shuffles, divides and powers; the
+// fused kernel's 16 warps per SM cannot hide their latency, while this kernel's few registers
+// and no CLT buffer let 64 warps share an SM.
+template <int NT>
+__device__ __forceinline__ void extract_task(const SceneDev &sc, const CorrConst &cfg, int quad, int RE, int task,
+                                             float *combo, int lane) {
+  const size_t tile = tile_of(sc, task);
+  float cmb[8], oprod[8];
+#pragma unroll
+  for (int t = 0; t < NT; t++) {
+    const int e = lane + 32 * t;
+    cmb[t] = (e < RE) ? sc.combo[tile * RE + e] : 0.f;
+  }
+  const float4 *ob = (const float4 *)(sc.osum + (tile * 32 + lane) * 8);
+  const float4 o0 = ob[0], o1 = ob[1];
+  oprod[0] = o0.x; oprod[1] = o0.y; oprod[2] = o0.z; oprod[3] = o0.w;
+  oprod[4] = o1.x; oprod[5] = o1.y; oprod[6] = o1.z; oprod[7] = o1.w;
+  const int ncomb = cfg.twice_diagonal ? 2 * cfg.num_combo : cfg.num_combo;
+  const float sum = fwd_extract_values<NT, true>(sc, cfg, quad, sc.num_pairs, RE, cfg.log_combine, ncomb, tile, combo,
+                                                 lane, cmb, oprod);
+  fwd_extract_finish(sc, cfg, quad, tile, combo, sum, lane);
+}
+
+template <int NT>
+__global__ void __launch_bounds__(128) extract_kernel(const __grid_constant__ SceneDev sc,
+                                                      const __grid_constant__ CorrConst cfg, int quad, int RE) {
+  __shared__ float s_combo[4][TP_MAX_STRIP * 15];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int task = blockIdx.x * 4 + warp;
+  if (task >= sc.num_tasks) return;  // whole warps
+  extract_task<NT>(sc, cfg, quad, RE, task, s_combo[warp], lane);
+}
+
+// the extraction of every scene of a batch: a block per unit of four tiles
+template <int NT>
+__global__ void __launch_bounds__(128) extract_batch_kernel(const SceneDev *__restrict__ scenes,
+                                                            const int *__restrict__ unit_off, int nscenes) {
+  __shared__ float s_combo[4][TP_MAX_STRIP * 15];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, u = blockIdx.x;
+  int lo = 0, hi = nscenes - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (unit_off[mid] <= u) lo = mid;
+    else hi = mid - 1;
+  }
+  const SceneDev &sc = scenes[lo];
+  const int task = (u - unit_off[lo]) * 4 + warp;
+  if (task >= sc.num_tasks) return;  // whole warps
+  const int RE = (sc.strip_rows < sc.wndy_size ? sc.strip_rows : sc.wndy_size) * 15;
+  extract_task<NT>(sc, *sc.corr_cfg, 1, RE, task, s_combo[warp], lane);
+}
+
+cudaError_t upload_quad_constants() { return upload_dtt_constants(); }
+
+static bool one_type(const SceneDev &sc) {
+  for (int i = 1; i < sc.num_sensors; i++)
+    if (sc.img_dtype[i] != sc.img_dtype[0]) return false;
+  return true;
+}
+
+// a standard quad with images of one type and room for the products between the two passes
+bool quad_forward_ok(const SceneDev &sc) { return sc.quad_std && sc.combo && sc.osum && one_type(sc); }
+
+// a batch's mono scenes, all standard quads of the same image type
+bool quad_batch_ok(const SceneDev *h, int n) {
+  for (int i = 0; i < n; i++)
+    if (!quad_forward_ok(h[i]) || h[i].num_colors != 1 || h[i].img_dtype[0] != h[0].img_dtype[0]) return false;
+  return n > 0;
+}
+
+cudaError_t launch_extract_pass(const SceneDev &sc, const CorrConst &cc, int quad, int RE, cudaStream_t st) {
+  if (RE <= 32) extract_kernel<1><<<(sc.num_tasks + 3) / 4, 128, 0, st>>>(sc, cc, quad, RE);
+  else extract_kernel<8><<<(sc.num_tasks + 3) / 4, 128, 0, st>>>(sc, cc, quad, RE);
+  return cudaGetLastError();
+}
+
+static int strip_entries(const SceneDev &sc) {
+  return (sc.strip_rows < sc.wndy_size ? sc.strip_rows : sc.wndy_size) * 15;
+}
+
+template <typename K>
+static cudaError_t go_quad(K kernel, int nw, const SceneDev &sc, const CorrConst &cc, int RE, cudaStream_t st) {
+  const int bytes = quad_warp_floats(sc.num_colors) * nw * 4, units = (sc.num_tasks + nw - 1) / nw;
+  int res = 0;
+  const cudaError_t e = kernel_residency((const void *)kernel, nw * 32, bytes, &res);
+  if (e != cudaSuccess) return e;
+  if (res < 1) return cudaErrorInvalidConfiguration;
+  kernel<<<units < res ? units : res, nw * 32, bytes, st>>>(sc, cc, RE);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_quad_forward(const SceneDev &sc, const CorrConst &cc, int nw, cudaStream_t st) {
+  const int RE = strip_entries(sc);
+  const bool one = RE <= 32, u16 = sc.img_dtype[0] == 1;
+  cudaError_t e;
+  if (sc.num_colors == 3) {
+    if (u16) e = one ? go_quad(quad_kernel<3, true, 1>, nw, sc, cc, RE, st) : go_quad(quad_kernel<3, true, 8>, nw, sc, cc, RE, st);
+    else e = one ? go_quad(quad_kernel<3, false, 1>, nw, sc, cc, RE, st) : go_quad(quad_kernel<3, false, 8>, nw, sc, cc, RE, st);
+  } else {
+    if (u16) e = one ? go_quad(quad_kernel<1, true, 1>, nw, sc, cc, RE, st) : go_quad(quad_kernel<1, true, 8>, nw, sc, cc, RE, st);
+    else e = one ? go_quad(quad_kernel<1, false, 1>, nw, sc, cc, RE, st) : go_quad(quad_kernel<1, false, 8>, nw, sc, cc, RE, st);
+  }
+  return e != cudaSuccess ? e : launch_extract_pass(sc, cc, 1, RE, st);
+}
+
+cudaError_t launch_quad_batch(const SceneDev *h, const SceneDev *scenes_dev, const int *unit_off_dev, int n,
+                              int total_units, cudaStream_t st) {
+  const int cf = (int)((offsetof(CorrConst, pairs) + 6 * sizeof(PairDev) + 15) / 16 * 4);
+  const int bytes = (cf + 4 * quad_warp_floats(1)) * 4;
+  bool one = true;
+  for (int i = 0; i < n; i++) one = one && strip_entries(h[i]) <= 32;
+  auto go = [&](auto kernel) -> cudaError_t {
+    int res = 0;
+    const cudaError_t e = kernel_residency((const void *)kernel, 128, bytes, &res);
+    if (e != cudaSuccess) return e;
+    if (res < 1) return cudaErrorInvalidConfiguration;
+    kernel<<<total_units < res ? total_units : res, 128, bytes, st>>>(scenes_dev, unit_off_dev, n, total_units, cf);
+    return cudaGetLastError();
+  };
+  cudaError_t e;
+  if (h[0].img_dtype[0] == 1) e = one ? go(quad_batch_kernel<true, 1>) : go(quad_batch_kernel<true, 8>);
+  else e = one ? go(quad_batch_kernel<false, 1>) : go(quad_batch_kernel<false, 8>);
+  if (e != cudaSuccess) return e;
+  if (one) extract_batch_kernel<1><<<total_units, 128, 0, st>>>(scenes_dev, unit_off_dev, n);
+  else extract_batch_kernel<8><<<total_units, 128, 0, st>>>(scenes_dev, unit_off_dev, n);
+  return cudaGetLastError();
+}
