@@ -604,6 +604,20 @@ static tp_status upload_geometry(tp_handle *h, const tp_geometry *g, const tp_ge
     gd.disp_num = rig->aux_disparity_radius;
     gd.disp_den = rig->main_disparity_radius;
   }
+  for (int s = 0; s < S; s++)
+    for (int i = 0; i < 3; i++) {
+      gd.rots_f[s][i] = gd.rots[s][i][2] * gd.fl_pix;
+      for (int k = 0; k < 4; k++) gd.drots_f[s][k][i] = gd.drots[s][k][i][2] * gd.fl_pix;
+      double d = 0.0;  // summed from 0 as the reference's matrix product
+      d += gd.rots[s][i][0] * -gd.rXY[s][0];
+      d += gd.rots[s][i][1] * -gd.rXY[s][1];
+      d += gd.rots[s][i][2] * 0.0;
+      gd.drot_disp[s][i] = d;
+    }
+  gd.n_rad = 7;
+  if (fabs(gd.ri_scale) < 1e10) {  // (not for an infinite or NaN scale, whose products the zero coefficients do not cancel)
+    while (gd.n_rad > 0 && g->distortion[gd.n_rad - 1] == 0.0) gd.n_rad--;
+  }
   std::vector<double> tbl;
   gd.tbl_len = host_rdist_table(gc, tbl);
   if (gd.tbl_len > 2048 + 64) return fail(h, TP_ERR_ARG, "distortion table too long");

@@ -43,6 +43,11 @@ struct GeomDev {
   double pXY0[TP_MAXS][2];
   double rots[TP_MAXS][3][3];
   double drots[TP_MAXS][4][3][3];
+  // products that are the same for every tile, taken once on the host (the same IEEE products)
+  double rots_f[TP_MAXS][3];      // rots[s][i][2] * fl_pix
+  double drots_f[TP_MAXS][4][3];  // drots[s][k][i][2] * fl_pix
+  double drot_disp[TP_MAXS][3];   // rots[s] x (-rX, -rY, 0)
+  int n_rad;                      // radial coefficients up to the last nonzero one
 };
 
 struct PairDev {

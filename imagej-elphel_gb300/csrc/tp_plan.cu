@@ -5,9 +5,13 @@
 // double precision with explicitly rounded operations (__dadd_rn etc. are never
 // contracted into FMAs) in the operation order of
 // GeometryCorrection.getPortsCoordinatesAndDerivatives and
-// ImageDtt.extract_correct_tile.  GB300 FP64 throughput is low, so this runs
-// as its own kernel with one thread per (task, sensor): ~100 FP64 operations
-// per port instead of the FP32 pipeline paying for them per coefficient.
+// ImageDtt.extract_correct_tile.  Two FP64 lanes per SM bound it at full size (an FP64 instruction
+// takes 64 issue slots), the chain of dependent FP64 instructions at small ones.  So what is exact in
+// integers (conversions, rounding to a corner, kernel centres) is done there, products that are the
+// same for every tile come with the geometry, zero radial coefficients are not evaluated, and small
+// task lists take a thread per (task, sensor).  Measured, before -> now: 4x2592x1936 Bayer with kernel
+// tables (78,408 tasks) 155 -> 65 us, 4x640x480 (4,800) 39 -> 11 us, 16x640x512 with derivatives 71 -> 43 us,
+// 16 batched 4x512x384 mono scenes 51 -> 23 us.
 #include "tp.h"
 #include "tp_internal.h"
 #include <math_constants.h>
@@ -45,79 +49,121 @@ __device__ double r_by_rdist(const double *tbl, int len, double rDist) {
   return DADD(tbl[index], DMUL(DSUB(tbl[index + 1], tbl[index]), DSUB(q, (double)index)));
 }
 
-__device__ __forceinline__ void mat3_vec(const double m[3][3], const double v[3], double r[3]) {
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    double s = 0.0;
-#pragma unroll
-    for (int k = 0; k < 3; k++) s = DADD(s, DMUL(m[i][k], v[k]));
-    r[i] = s;
-  }
+// Exact conversions by bit assembly.  FP64 instructions (conversions among them) issue at 1/64 of
+// the integer rate here and bound this file's kernels, so everything that is exact in integers stays
+// there.
+__device__ __forceinline__ double f2d(float f) {
+  const unsigned u = __float_as_uint(f), e = (u >> 23) & 255u;
+  if (e - 1u < 254u)  // normal
+    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))), (int)(u << 29));
+  if ((u << 1) == 0u) return __hiloint2double((int)u, 0);
+  return (double)f;
+}
+__device__ __forceinline__ double i2d(int n) { return (n < (1 << 24) && n > -(1 << 24)) ? f2d((float)n) : (double)n; }
+// n / 2 (n = 0: 0)
+__device__ __forceinline__ double half_i2d(int n) {
+  const double d = i2d(n);
+  return n ? __hiloint2double(__double2hiint(d) - (1 << 20), __double2loint(d)) : 0.0;
+}
+// java_round(x / 2^k) as an integer for |x| < 2^30: floor(2 x / 2^k) is an arithmetic shift of the
+// signed mantissa, and java_round(y) = (floor(2 y) + 1) >> 1.  Returns false (n unset) beyond, and for NaN.
+__device__ __forceinline__ bool jround(double x, int k, int &n) {
+  const int hi = __double2hiint(x), e = ((hi >> 20) & 0x7ff) - 1023;
+  if (e >= 30) return false;
+  const long long m = ((long long)((hi & 0xfffff) | 0x100000) << 32) | (unsigned)__double2loint(x);
+  const int sh = min(51 - e + k, 63);
+  n = (int)((((hi < 0 ? -m : m) >> sh) + 1) >> 1);
+  return true;
 }
 
 // undistorted tile centre, the sensor-independent head of getPortsCoordinatesAndDerivatives, with
-// the centre model (gc_main, 2179-2185)
-__device__ __forceinline__ void center_undistort(const GeomDev &g, const double *tbl, double px, double py,
-                                                 double &pXc, double &pYc) {
-  const double pXcd = DSUB(px, DMUL(0.5, (double)g.c_pixel_width));
-  const double pYcd = DSUB(py, DMUL(0.5, (double)g.c_pixel_height));
+// the centre model (gc_main, 2179-2185); px, py: the centre (2 px - width is exact in integers)
+__device__ __forceinline__ void center_undistort(const GeomDev &g, const double *tbl, int px, int py, double &pXc,
+                                                 double &pYc) {
+  const double pXcd = half_i2d(2 * px - g.c_pixel_width);
+  const double pYcd = half_i2d(2 * py - g.c_pixel_height);
   const double rD = DMUL(DMUL(DSQRT(DADD(DMUL(pXcd, pXcd), DMUL(pYcd, pYcd))), 0.001), g.c_pixel_size);
   const double rND2R = r_by_rdist(tbl, g.tbl_len, DDIV(rD, g.c_distortion_radius));
   pXc = DMUL(pXcd, rND2R);
   pYc = DMUL(pYcd, rND2R);
 }
 
-// getPortsCoordinatesAndDerivatives (GeometryCorrection.java:2159-2314) for one sensor
-// (pXc, pYc): the task's undistorted centre (center_undistort), the same for every sensor
-__device__ void port_xy(const GeomDev &g, double pXc, double pYc, double disparity, int i, double &ox, double &oy,
-                        double *deriv /* [2][5] or null */) {
-  const double fl_pix = g.fl_pix, ri_scale = g.ri_scale;
-  double vi[3] = {DSUB(pXc, DMUL(disparity, g.rXY[i][0])), DSUB(pYc, DMUL(disparity, g.rXY[i][1])), fl_pix};
-  double rvi[3];
-  mat3_vec(g.rots[i], vi, rvi);
-  double norm_z = DDIV(fl_pix, rvi[2]);
-  double pXci = DMUL(rvi[0], norm_z);
-  double pYci = DMUL(rvi[1], norm_z);
-  double rNDi = DSQRT(DADD(DMUL(pXci, pXci), DMUL(pYci, pYci)));
-  double ri = DMUL(rNDi, ri_scale);
-  double rD2rND = 1.0, rri = 1.0;
-#pragma unroll
-  for (int j = 0; j < 7; j++) {
-    rri = DMUL(rri, ri);
-    rD2rND = DADD(rD2rND, DMUL(g.rad_coeff[j], DSUB(rri, 1.0)));
+// A rotation times (v0, v1, fl_pix): the third product is the same for every tile and comes with the
+// geometry (m2f[i] = m[i][2] * fl_pix), summed last as in the reference's matrix product.
+__device__ __forceinline__ double row_vec(const double m[3], double m2f, double v0, double v1) {
+  return DADD(DADD(DMUL(m[0], v0), DMUL(m[1], v1)), m2f);
+}
+
+// sensor part of getPortsCoordinatesAndDerivatives (GeometryCorrection.java:2159-2314) for one sensor;
+// (pXc, pYc): the task's undistorted centre, the same for every sensor.  The radial polynomial runs to
+// the last nonzero coefficient only (g.n_rad): a zero one adds 0 x (a finite number).  Where that
+// number would not be finite (pXci or pYci out of range or NaN), or the radius is 0 (its derivatives are
+// then NaN), all seven are taken.
+template <bool DERIV>
+__device__ __forceinline__ void sensor_port(const GeomDev &g, double pXc, double pYc, double disparity, int i,
+                                            double &ox, double &oy, double *deriv /* [2][5] */) {
+  const double fl_pix = g.fl_pix;
+  const double v0 = DSUB(pXc, DMUL(disparity, g.rXY[i][0])), v1 = DSUB(pYc, DMUL(disparity, g.rXY[i][1]));
+  const double r0 = row_vec(g.rots[i][0], g.rots_f[i][0], v0, v1);
+  const double r1 = row_vec(g.rots[i][1], g.rots_f[i][1], v0, v1);
+  const double r2 = row_vec(g.rots[i][2], g.rots_f[i][2], v0, v1);
+  const double norm_z = DDIV(fl_pix, r2);
+  const double pXci = DMUL(r0, norm_z), pYci = DMUL(r1, norm_z);
+  const int lim = (1023 + 100) << 20;  // 2^100
+  const int hx = __double2hiint(pXci) & 0x7fffffff, hy = __double2hiint(pYci) & 0x7fffffff;
+  const int n_rad = (hx < lim && hy < lim && (hx | hy)) ? g.n_rad : 7;
+  double rD2rND = 1.0, ri = 0.0, rNDi = 0.0;
+  if (n_rad) {
+    rNDi = DSQRT(DADD(DMUL(pXci, pXci), DMUL(pYci, pYci)));
+    ri = DMUL(rNDi, g.ri_scale);
+    double rri = 1.0;
+    for (int j = 0; j < n_rad; j++) {
+      rri = DMUL(rri, ri);
+      rD2rND = DADD(rD2rND, DMUL(g.rad_coeff[j], DSUB(rri, 1.0)));
+    }
+    ox = DADD(DMUL(pXci, rD2rND), g.pXY0[i][0]);
+    oy = DADD(DMUL(pYci, rD2rND), g.pXY0[i][1]);
+  } else {
+    ox = DADD(pXci, g.pXY0[i][0]);
+    oy = DADD(pYci, g.pXY0[i][1]);
   }
-  ox = DADD(DMUL(pXci, rD2rND), g.pXY0[i][0]);
-  oy = DADD(DMUL(pYci, rD2rND), g.pXY0[i][1]);
-  if (deriv) {
+  if constexpr (DERIV) {
     // quotients shared by the five parameters (a product with a reciprocal where the reference
     // divides: the derivatives differ from its by an ulp, the ports are not touched)
-    const double ri_rnd = DDIV(ri_scale, rNDi);
-    const double inv_rz = DDIV(1.0, rvi[2]);
+    const double inv_rz = DDIV(1.0, r2);
     const double pXr = DMUL(pXci, inv_rz), pYr = DMUL(pYci, inv_rz);
-    double drD2rND_dri = 0.0;
-    rri = 1.0;
-#pragma unroll
-    for (int j = 0; j < 7; j++) {
-      drD2rND_dri = DADD(drD2rND_dri, DMUL(g.rad_dcoeff[j], rri));
-      rri = DMUL(rri, ri);
+    double ri_rnd = 0.0, drD2rND_dri = 0.0;
+    if (n_rad) {
+      ri_rnd = DDIV(g.ri_scale, rNDi);
+      double rri = 1.0;
+      for (int j = 0; j < n_rad; j++) {
+        drD2rND_dri = DADD(drD2rND_dri, DMUL(g.rad_dcoeff[j], rri));
+        rri = DMUL(rri, ri);
+      }
     }
 #pragma unroll
     for (int k = 0; k < 5; k++) {  // azimuth, tilt, roll, zoom; then the tile disparity
-      double dr[3];
+      double d0, d1, d2;
       if (k < 4) {
-        mat3_vec(g.drots[i][k], vi, dr);
-      } else {  // d vi / d disparity = (-rX, -rY, 0)
-        const double dvi[3] = {-g.rXY[i][0], -g.rXY[i][1], 0.0};
-        mat3_vec(g.rots[i], dvi, dr);
+        d0 = row_vec(g.drots[i][k][0], g.drots_f[i][k][0], v0, v1);
+        d1 = row_vec(g.drots[i][k][1], g.drots_f[i][k][1], v0, v1);
+        d2 = row_vec(g.drots[i][k][2], g.drots_f[i][k][2], v0, v1);
+      } else {  // d (v0, v1, fl_pix) / d disparity = (-rX, -rY, 0), rotated
+        d0 = g.drot_disp[i][0];
+        d1 = g.drot_disp[i][1];
+        d2 = g.drot_disp[i][2];
       }
-      double dpX = DSUB(DMUL(dr[0], norm_z), DMUL(pXr, dr[2]));
-      double dpY = DSUB(DMUL(dr[1], norm_z), DMUL(pYr, dr[2]));
-      if (k == 2) {  // roll: the reference keeps only the rotation term
+      const double dpX = DSUB(DMUL(d0, norm_z), DMUL(pXr, d2));
+      const double dpY = DSUB(DMUL(d1, norm_z), DMUL(pYr, d2));
+      if (!n_rad) {
+        deriv[k] = dpX;
+        deriv[5 + k] = dpY;
+      } else if (k == 2) {  // roll: the reference keeps only the rotation term
         deriv[k] = DMUL(dpX, rD2rND);
         deriv[5 + k] = DMUL(dpY, rD2rND);
       } else {
-        double dri = DMUL(ri_rnd, DADD(DMUL(pXci, dpX), DMUL(pYci, dpY)));
-        double drD = DMUL(drD2rND_dri, dri);
+        const double dri = DMUL(ri_rnd, DADD(DMUL(pXci, dpX), DMUL(pYci, dpY)));
+        const double drD = DMUL(drD2rND_dri, dri);
         deriv[k] = DADD(DMUL(dpX, rD2rND), DMUL(pXci, drD));
         deriv[5 + k] = DADD(DMUL(dpY, rD2rND), DMUL(pYci, drD));
       }
@@ -125,107 +171,104 @@ __device__ void port_xy(const GeomDev &g, double pXc, double pYc, double dispari
   }
 }
 
-// sensor part of getPortsCoordinatesAndDerivatives (GeometryCorrection.java:2190-2217)
-__device__ __forceinline__ void sensor_port(const GeomDev &g, double pXc, double pYc, double disparity, int i,
-                                            double &ox, double &oy) {
-  const double fl_pix = g.fl_pix, ri_scale = g.ri_scale;
-  const double vi[3] = {DSUB(pXc, DMUL(disparity, g.rXY[i][0])), DSUB(pYc, DMUL(disparity, g.rXY[i][1])), fl_pix};
-  double rvi[3];
-  mat3_vec(g.rots[i], vi, rvi);
-  const double norm_z = DDIV(fl_pix, rvi[2]);
-  const double pXci = DMUL(rvi[0], norm_z), pYci = DMUL(rvi[1], norm_z);
-  const double ri = DMUL(DSQRT(DADD(DMUL(pXci, pXci), DMUL(pYci, pYci))), ri_scale);
-  double rD2rND = 1.0, rri = 1.0;
-#pragma unroll
-  for (int j = 0; j < 7; j++) {
-    rri = DMUL(rri, ri);
-    rD2rND = DADD(rD2rND, DMUL(g.rad_coeff[j], DSUB(rri, 1.0)));
+// window corner and residual shift along one axis (ImageDtt.java:4940-4943) from px = the window's
+// exact corner: TL = -java_round(-px), residual = -(px - TL)
+__device__ __forceinline__ void corner(double px, int n, int &tl, float &res) {
+  int m;
+  if (jround(-px, 0, m)) {
+    const int lo = -(TP_PORT_MARGIN + 16), hi = n + TP_PORT_MARGIN;
+    tl = -m;
+    res = (float)(-DSUB(px, i2d(tl)));
+    if (tl < lo || tl > hi) {  // clamp_corner
+      const int par = tl & 1;
+      tl = (tl > hi) ? hi - ((hi & 1) ^ par) : lo + ((lo & 1) ^ par);
+    }
+  } else {  // beyond +-2^30 pixels, or NaN
+    const double t = -java_round(-px);
+    tl = clamp_corner(t, n);
+    res = (float)(-DSUB(px, t));
   }
-  ox = DADD(DMUL(pXci, rD2rND), g.pXY0[i][0]);
-  oy = DADD(DMUL(pYci, rD2rND), g.pXY0[i][1]);
 }
 
-// One thread per task: the centre is undistorted once, the kernel tile is found
-// once per sensor (it depends on the port only), then each colour's window
-// corner and residual shift (ImageDtt.java:4904-4943).  A division by a
-// power-of-two kernel step is replaced by the multiplication with its exact
-// reciprocal, which IEEE rounding makes bit-identical.
+// kernel tile along one axis: round(c / ks) + 1 within the table, and the distance from its centre
+__device__ __forceinline__ int kernel_tile(double c, int ks, int ks_log2, int nk, double &d) {
+  int m;
+  if (ks_log2 < 0 || !jround(c, ks_log2, m)) m = (int)java_round(DDIV(c, (double)ks));
+  int kt = m + 1;
+  kt = kt < 0 ? 0 : (kt >= nk ? nk - 1 : kt);
+  // ((kt - 1) + 0.5) * ks
+  const long long c2 = (2ll * kt - 1) * ks;
+  d = DSUB(c, (c2 < (1 << 30) && c2 > -(1 << 30)) ? half_i2d((int)c2) : DMUL(DADD((double)(kt - 1), 0.5), (double)ks));
+  return kt;
+}
+
+// Thread per (task, run of sensors): the centre is undistorted once per thread, the kernel tile
+// found once per sensor (it depends on the port only), then each colour's window corner and residual
+// shift (ImageDtt.java:4904-4943).
 // sensors [s0, s1) of one task
+template <bool DERIV>
 __device__ __forceinline__ void plan_task(const SceneDev &sc, int task, int s0, int s1) {
   const int S = sc.num_sensors, C = sc.num_colors;
   const int txy = sc.task_txy[task];
   const int tx = txy & 0xffff, ty = txy >> 16;
-  const double ctx = (double)(tx * TP_DTT + TP_DTT / 2), cty = (double)(ty * TP_DTT + TP_DTT / 2);
   double pXc = 0.0, pYc = 0.0, disparity = 0.0;
   if (sc.ports_from_geometry) {
-    center_undistort(*sc.geom, sc.rdist_tbl, ctx, cty, pXc, pYc);
-    disparity = (double)sc.task_disp[task];
+    center_undistort(*sc.geom, sc.rdist_tbl, tx * TP_DTT + TP_DTT / 2, ty * TP_DTT + TP_DTT / 2, pXc, pYc);
+    disparity = f2d(sc.task_disp[task]);
     // a rig's auxiliary camera: disparity_main * aux radius / main radius (ImageDtt.java:8973)
     if (sc.geom->rig) disparity = DDIV(DMUL(disparity, sc.geom->disp_num), sc.geom->disp_den);
   }
   const int ks = sc.kernel_step;
-  const bool pow2 = ks > 0 && (ks & (ks - 1)) == 0;
-  const double inv_ks = pow2 ? 1.0 / (double)ks : 0.0;
+  const int ks_log2 = (ks > 0 && (ks & (ks - 1)) == 0) ? 31 - __clz(ks) : -1;
   for (int s = s0; s < s1; s++) {
     double cx, cy;
     if (sc.ports_from_geometry) {
-      if (sc.port_deriv) {
-        double dv[10];
-        port_xy(*sc.geom, pXc, pYc, disparity, s, cx, cy, dv);
+      double dv[10];
+      sensor_port<DERIV>(*sc.geom, pXc, pYc, disparity, s, cx, cy, dv);
+      if constexpr (DERIV) {
         double *o = sc.port_deriv + ((size_t)task * S + s) * 10;
 #pragma unroll
         for (int k = 0; k < 10; k++) o[k] = dv[k];
-      } else {
-        sensor_port(*sc.geom, pXc, pYc, disparity, s, cx, cy);
       }
     } else {
-      cx = (double)sc.task_xy[((size_t)task * S + s) * 2];
-      cy = (double)sc.task_xy[((size_t)task * S + s) * 2 + 1];
+      cx = f2d(sc.task_xy[((size_t)task * S + s) * 2]);
+      cy = f2d(sc.task_xy[((size_t)task * S + s) * 2 + 1]);
     }
     sc.ports[((size_t)task * S + s) * 2] = cx;
     sc.ports[((size_t)task * S + s) * 2 + 1] = cy;
     int ktx = 0, kty = 0;
     double kdx = 0.0, kdy = 0.0;
     if (sc.kh > 0) {
-      const double qx = pow2 ? DMUL(cx, inv_ks) : DDIV(cx, (double)ks);
-      const double qy = pow2 ? DMUL(cy, inv_ks) : DDIV(cy, (double)ks);
-      ktx = (int)java_round(qx) + 1;
-      kty = (int)java_round(qy) + 1;
-      kty = kty < 0 ? 0 : (kty >= sc.kv ? sc.kv - 1 : kty);
-      ktx = ktx < 0 ? 0 : (ktx >= sc.kh ? sc.kh - 1 : ktx);
-      kdx = DSUB(cx, DMUL(DADD((double)(ktx - 1), 0.5), (double)ks));
-      kdy = DSUB(cy, DMUL(DADD((double)(kty - 1), 0.5), (double)ks));
+      ktx = kernel_tile(cx, ks, ks_log2, sc.kh, kdx);
+      kty = kernel_tile(cy, ks, ks_log2, sc.kv, kdy);
     }
+    const double cx8 = DSUB(cx, (double)TP_DTT), cy8 = DSUB(cy, (double)TP_DTT);
     for (int c = 0; c < C; c++) {
-      double px = DSUB(cx, (double)TP_DTT), py = DSUB(cy, (double)TP_DTT);
-      int kidx = -1;
-      if (sc.kh > 0) {
-        kidx = (kty * sc.kh + ktx) * C + c;
-        const float4 *ce4 = (const float4 *)(sc.kext[s] + (size_t)kidx * 8);
-        const float4 e0 = __ldg(ce4), e1 = __ldg(ce4 + 1);  // data_x, data_y, -, -, dxc_dx, dxc_dy, dyc_dx, dyc_dy
-        px = DSUB(DSUB(cx, (double)TP_DTT), DADD(DADD((double)e0.x, DMUL((double)e1.x, kdx)), DMUL((double)e1.y, kdy)));
-        py = DSUB(DSUB(cy, (double)TP_DTT), DADD(DADD((double)e0.y, DMUL((double)e1.z, kdx)), DMUL((double)e1.w, kdy)));
-      }
-      const double tl = -java_round(-px), tt = -java_round(-py);
+      double px = cx8, py = cy8;
       SubtilePlan p;
-      p.tlx = clamp_corner(tl, sc.width);
-      p.tly = clamp_corner(tt, sc.height);
-      p.kidx = kidx;
-      p.rx = (float)(-(DSUB(px, tl)));
-      p.ry = (float)(-(DSUB(py, tt)));
+      p.kidx = -1;
+      if (sc.kh > 0) {
+        p.kidx = (kty * sc.kh + ktx) * C + c;
+        const float4 *ce4 = (const float4 *)(sc.kext[s] + (size_t)p.kidx * 8);
+        const float4 e0 = __ldg(ce4), e1 = __ldg(ce4 + 1);  // data_x, data_y, -, -, dxc_dx, dxc_dy, dyc_dx, dyc_dy
+        px = DSUB(px, DADD(DADD(f2d(e0.x), DMUL(f2d(e1.x), kdx)), DMUL(f2d(e1.y), kdy)));
+        py = DSUB(py, DADD(DADD(f2d(e0.y), DMUL(f2d(e1.z), kdx)), DMUL(f2d(e1.w), kdy)));
+      }
+      corner(px, sc.width, p.tlx, p.rx);
+      corner(py, sc.height, p.tly, p.ry);
       sc.plan[((size_t)task * S + s) * C + c] = p;
     }
   }
 }
 
-// thread per (task, group of up to 4 sensors): 16-sensor scenes get 4x the threads
-__global__ void plan_kernel(SceneDev sc) {
-  const int groups = (sc.num_sensors + 3) >> 2;
+// gs sensors per thread
+template <bool DERIV>
+__global__ void plan_kernel(SceneDev sc, int gs) {
+  const int groups = (sc.num_sensors + gs - 1) / gs;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= sc.num_tasks * groups) return;
-  const int task = i / groups, g = i - task * groups;
-  const int s0 = g * 4, s1 = (s0 + 4 < sc.num_sensors) ? s0 + 4 : sc.num_sensors;
-  plan_task(sc, task, s0, s1);
+  const int task = i / groups, s0 = (i - task * groups) * gs;
+  plan_task<DERIV>(sc, task, s0, min(s0 + gs, sc.num_sensors));
 }
 
 // the plans of a batch of scenes in one launch: thread per task of the
@@ -241,7 +284,7 @@ __global__ void plan_batch_kernel(const SceneDev *__restrict__ scenes, const int
   }
   const SceneDev &sc = scenes[lo];
   const int task = g - task_off[lo];
-  plan_task(sc, task, 0, sc.num_sensors);
+  plan_task<false>(sc, task, 0, sc.num_sensors);
   const int txy = sc.task_txy[task];
   sc.tile_task[(txy >> 16) * sc.tilesX + (txy & 0xffff)] = task;
 }
@@ -297,10 +340,16 @@ __global__ void compact_tasks_kernel(const int *tile_op, const float *disparity,
   if (threadIdx.x == 0) *num_tasks = base;
 }
 
+// Sensors per thread: with few threads the kernel is a chain of dependent FP64 instructions, so each
+// takes one sensor; with many the FP64 pipes are full, and four sensors share the centre's part.
+// The line: about one warp per scheduler (32 x 4 x 152 threads).
 cudaError_t launch_plan(const SceneDev &sc, cudaStream_t st) {
-  const int n = sc.num_tasks * ((sc.num_sensors + 3) / 4);
-  if (n <= 0) return cudaSuccess;
-  plan_kernel<<<(n + 63) / 64, 64, 0, st>>>(sc);
+  if (sc.num_tasks <= 0) return cudaSuccess;
+  int gs = 1;
+  while (gs < 4 && sc.num_tasks * ((sc.num_sensors + gs - 1) / gs) > 32 * 4 * 152) gs *= 2;
+  const int n = sc.num_tasks * ((sc.num_sensors + gs - 1) / gs);
+  if (sc.port_deriv && sc.ports_from_geometry) plan_kernel<true><<<(n + 63) / 64, 64, 0, st>>>(sc, gs);
+  else plan_kernel<false><<<(n + 63) / 64, 64, 0, st>>>(sc, gs);
   return cudaGetLastError();
 }
 
