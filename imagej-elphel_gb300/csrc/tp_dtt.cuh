@@ -169,6 +169,7 @@ __device__ __forceinline__ void fold_dtt_dense(const PIX &w, const FoldIdx &fv, 
     p0[cix] = w.at(fv.src0, cix);
     p1[cix] = w.at(fv.src1, cix);
   }
+  __syncwarp();  // every window is read: the transpose buffers may lie over them
   // vertical 2-tap combine once, then the two horizontal variants
 #pragma unroll
   for (int vb = 0; vb < 2; vb++) {

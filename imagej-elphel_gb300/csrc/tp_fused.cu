@@ -755,6 +755,7 @@ cudaError_t launch_fused_forward(const SceneDev &sc, const CorrConst &cc, int tp
   }
   FwdShape f = make_shape(sc, nw);
   if (f.nw > 4) return cudaErrorInvalidConfiguration;
+  if (tpb == 1 && f.nw == 4 && many_forward_ok(sc)) return launch_many_forward(sc, cc, st);
   if (tpb == 1 && f.nw > 1) {
     const int bytes = split_smem_floats(f) * 4;
     if (f.nw == 3) {  // quad colour scenes: one colour item per warp, 8 CTAs per SM

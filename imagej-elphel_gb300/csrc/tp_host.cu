@@ -234,6 +234,8 @@ static SceneDev scene_of(tp_handle *h) {
   sc.num_pairs = h->num_pairs;
   sc.strip_rows = h->corr_host.strip_rows;
   sc.wndy_size = h->corr_host.wndy_size;
+  sc.all_general = h->num_pairs > 0;
+  for (int i = 0; i < h->num_pairs; i++) sc.all_general &= h->corr_host.pairs[i].kind == 4;
   sc.quad_std = is_standard_quad(h);
   return sc;
 }
@@ -448,6 +450,7 @@ tp_status tp_create(const tp_config *cfg, tp_handle **out) {
   ok = ok && upload_kernel_constants() == cudaSuccess;
   ok = ok && upload_fused_constants() == cudaSuccess;
   ok = ok && upload_quad_constants() == cudaSuccess;
+  ok = ok && upload_many_constants() == cudaSuccess;
   ok = ok && upload_texture_constants() == cudaSuccess;
   ok = ok && upload_adjoint_constants() == cudaSuccess;
   ok = ok && upload_kernprep_constants() == cudaSuccess;
@@ -953,6 +956,27 @@ tp_status tp_set_corr(tp_handle *h, const tp_corr_params *p, const tp_pair *pair
         }
         cd.strip_code[kind][e][dn] = code;
       }
+  // strip taps of general pairs (strip_sample, the same FP32 operations)
+  for (int i = 0; i < np; i++)
+    for (int e = 0; e < 32; e++) {
+      int cells = 0;
+      for (int side = 0; side < 2; side++) {
+        const int row = e / 15, scol = e % 15 - 7, down = side ? 1 : -1;
+        const float bx = cd.pairs[i].bx, by = cd.pairs[i].by;
+        const float a = scol + 0.5f * (row & 1), pp = 0.5f * down * row;
+        const float x = fmaf(-pp, by, a * bx), y = fmaf(pp, bx, a * by);
+        if (!(x <= 7.f && x >= -7.f && y <= 7.f && y >= -7.f)) {
+          cells |= 1 << (16 + side);
+          continue;
+        }
+        const float fx = x + 7.f, fy = y + 7.f;
+        const int ix0 = (int)fx < 13 ? (int)fx : 13, iy0 = (int)fy < 13 ? (int)fy : 13;
+        cd.gen_tap[i][e][2 * side] = fx - ix0;
+        cd.gen_tap[i][e][2 * side + 1] = fy - iy0;
+        cells |= (iy0 * 15 + ix0) << (8 * side);
+      }
+      cd.gen_cell[i][e] = cells;
+    }
   // the adjoint's rounds: greedily, in pair order, up to 4 combined-strip pairs on distinct sensors
   {
     std::vector<int> left;

@@ -87,6 +87,11 @@ struct CorrDev : CorrConst {
   // sensors are all distinct, so the four warps of a tile add their pairs' CLT gradients into
   // disjoint sensors, and every sensor's gradient is summed in the same pair order in every run
   short adj_round[TP_MAXP][4];
+  // strip taps of general pairs (kind 4) for the first 32 strip entries: the bilinear fractions of the two
+  // sides (x, y below; x, y above) and the cells, 8 bits a side, bit 16 / 17 set where a side falls
+  // outside the surface.  They are the same for every tile.
+  alignas(16) float gen_tap[TP_MAXP][32][4];
+  int gen_cell[TP_MAXP][32];
 };
 
 struct SceneDev {
@@ -129,6 +134,7 @@ struct SceneDev {
   int num_pairs;             // host copy of corr_cfg->num_pairs (launch sizing)
   int strip_rows;            // host copy of corr_cfg->strip_rows
   int wndy_size;             // host copy of corr_cfg->wndy_size
+  int all_general;           // every pair is of kind 4 (the many-pair kernel's strip taps apply)
   int quad_std;              // the pairs are the six of a standard quad, in its order (is_standard_quad)
 };
 
@@ -169,6 +175,10 @@ cudaError_t launch_quad_forward(const SceneDev &sc, const CorrConst &cc, int nw,
 bool quad_batch_ok(const SceneDev *scenes_host, int n);
 cudaError_t launch_quad_batch(const SceneDev *scenes_host, const SceneDev *scenes_dev, const int *unit_off_dev, int n,
                               int total_units, cudaStream_t st);
+// mono scenes with many general pairs (tp_many.cu)
+cudaError_t upload_many_constants();
+bool many_forward_ok(const SceneDev &sc);
+cudaError_t launch_many_forward(const SceneDev &sc, const CorrConst &cc, cudaStream_t st);
 // phase C of a forward that left its strip and ortho profile products in sc.combo and sc.osum
 cudaError_t launch_extract_pass(const SceneDev &sc, const CorrConst &cc, int quad, int RE, cudaStream_t st);
 // GPU_DTT24_DRV counterpart (tp_fused.cu): 2D DTT of one mode on every 8x8 block

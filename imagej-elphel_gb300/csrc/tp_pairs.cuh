@@ -67,6 +67,16 @@ __device__ __forceinline__ void warp_sum6(const float v[6], int lane, float k0, 
   for (int p = 0; p < 6; p++) out[p] = __shfl_sync(0xffffffffu, t, (p / 3) * 16 + ((p % 3) == 0 ? 0 : ((p % 3) == 1 ? 4 : 8)));
 }
 
+// the same for two values: sums of a over lanes and of b over lanes, each times k0 and fz
+__device__ __forceinline__ float2 warp_sum2(float2 v, int lane, float k0, float fz) {
+  const bool h16 = lane & 16;
+  float t = (h16 ? v.y : v.x) + __shfl_xor_sync(0xffffffffu, h16 ? v.x : v.y, 16);
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  t = t * k0 * fz;
+  return make_float2(__shfl_sync(0xffffffffu, t, 0), __shfl_sync(0xffffffffu, t, 16));
+}
+
 // the normalised products of a pair (Correlation2d.correlateSingleColorFD, the ZI table) on two
 // CLT indices: t[0..3] from a (first sensor), its negatives n[1..3] and b (second sensor)
 __device__ __forceinline__ void clt_products(const float2 a[4], const float2 n[4], const float2 b[4], float2 t[4]) {

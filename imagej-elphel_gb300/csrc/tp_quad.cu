@@ -212,10 +212,12 @@ __device__ __forceinline__ void extract_task(const SceneDev &sc, const CorrConst
     const int e = lane + 32 * t;
     cmb[t] = (e < RE) ? sc.combo[tile * RE + e] : 0.f;
   }
-  const float4 *ob = (const float4 *)(sc.osum + (tile * 32 + lane) * 8);
-  const float4 o0 = ob[0], o1 = ob[1];
-  oprod[0] = o0.x; oprod[1] = o0.y; oprod[2] = o0.z; oprod[3] = o0.w;
-  oprod[4] = o1.x; oprod[5] = o1.y; oprod[6] = o1.z; oprod[7] = o1.w;
+  if (quad) {  // other layouts have no ortho profiles
+    const float4 *ob = (const float4 *)(sc.osum + (tile * 32 + lane) * 8);
+    const float4 o0 = ob[0], o1 = ob[1];
+    oprod[0] = o0.x; oprod[1] = o0.y; oprod[2] = o0.z; oprod[3] = o0.w;
+    oprod[4] = o1.x; oprod[5] = o1.y; oprod[6] = o1.z; oprod[7] = o1.w;
+  }
   const int ncomb = cfg.twice_diagonal ? 2 * cfg.num_combo : cfg.num_combo;
   const float sum = fwd_extract_values<NT, true>(sc, cfg, quad, sc.num_pairs, RE, cfg.log_combine, ncomb, tile, combo,
                                                  lane, cmb, oprod);
