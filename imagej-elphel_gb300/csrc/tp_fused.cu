@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(MAXT, MINB) fused_split_kernel(const __grid_co
 // shared memory (reloaded only when the scene changes); the scene's
 // correlation set-up is read through its device pointer.
 // ---------------------------------------------------------------------------
-__global__ void disp_init_kernel(float *disp, int n);
+static cudaError_t init_records(const SceneDev &sc, cudaStream_t st);
 
 int batch_class(const SceneDev &sc) {
   if (sc.num_colors == 3) return 0;
@@ -387,8 +387,8 @@ cudaError_t launch_fused_batch(int cls, const SceneDev *scenes_host, const Scene
     maxre = re > maxre ? re : maxre;
     const SceneDev &sc = scenes_host[i];
     if (batch_class(sc) != cls || sc.strip_rows * 15 > 8 * 32) return cudaErrorInvalidValue;
-    const int ntiles = sc.tilesX * sc.tilesY;
-    disp_init_kernel<<<(ntiles * TP_NDISP + 255) / 256, 256, 0, st>>>(sc.disp, ntiles);
+    const cudaError_t ei = init_records(sc, st);
+    if (ei != cudaSuccess) return ei;
     const int f = ((sc.num_sensors * sc.num_colors * TP_CLT + SCR) + 3) & ~3;
     wf = f > wf ? f : wf;
     const int g = sc.num_sensors * TP_CLT + 4 * SCR + 4 * 240;
@@ -664,6 +664,15 @@ __global__ void disp_init_kernel(float *disp, int n) {
   }
 }
 
+// The records of tiles outside the task list; a forward writes all of its tasks' records, so where a
+// task list made from tile ops (no tile twice) holds every tile there is nothing to do.
+static cudaError_t init_records(const SceneDev &sc, cudaStream_t st) {
+  const int ntiles = sc.tilesX * sc.tilesY;
+  if (sc.ports_from_geometry && sc.num_tasks == ntiles) return cudaSuccess;
+  disp_init_kernel<<<(ntiles * TP_NDISP + 255) / 256, 256, 0, st>>>(sc.disp, ntiles);
+  return cudaGetLastError();
+}
+
 cudaError_t upload_fused_constants() { return upload_dtt_constants(); }
 
 // GPU_DTT24_DRV (dtt8x8.cuh:100-158): every 8x8 block of a float image through the 2D transform of
@@ -744,9 +753,7 @@ static cudaError_t launch_persistent(K kernel, int threads, int bytes, int units
 // Schedules: tiles_per_block == warps_per_block (<= 4): warp per tile;
 // tiles_per_block == 1 with warps_per_block 2, 3 or 4: pair per warp (CTA per tile).
 cudaError_t launch_fused_forward(const SceneDev &sc, const CorrConst &cc, int tpb, int nw, cudaStream_t st) {
-  const int ntiles = sc.tilesX * sc.tilesY;
-  disp_init_kernel<<<(ntiles * TP_NDISP + 255) / 256, 256, 0, st>>>(sc.disp, ntiles);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = init_records(sc, st);
   if (e != cudaSuccess || sc.num_tasks <= 0) return e;
   if (sc.strip_rows * 15 > 8 * 32) return cudaErrorInvalidConfiguration;
   if (tpb <= 0 && nw <= 0 && sc.num_pairs > 8) {  // default for many pairs: four warps share a tile

@@ -23,6 +23,7 @@ struct tp_handle {
   cudaStream_t stream = nullptr;
   // recorded on the stream of every call that enqueues work; the getters' copies wait for it
   cudaEvent_t ev_work = nullptr;
+  cudaStream_t work_st = nullptr;  // the stream ev_work was recorded on last
   std::string err;
   // device buffers
   void *d_images[TP_MAXS] = {};
@@ -57,8 +58,7 @@ struct tp_handle {
   int rig_lma_done = 0;        // the rig record already holds the LMA branch's values
   // page-locked copies of the last tile ops / disparities (tp_set_tile_ops returns before its
   // upload runs), reused once the event after their upload has passed
-  int *h_stage_op = nullptr;
-  float *h_stage_disp = nullptr;
+  int *h_stage_op = nullptr;  // page-locked [2][tiles]: tile ops, then disparities
   cudaEvent_t ev_stage = nullptr;
   float *d_lma = nullptr;    // [tiles][4] LMA disparity, strength, WM, WXY
   float *d_mismatch = nullptr;  // [tiles][pairs][3] lazy-eye mismatch of the last LMA pass that measured it
@@ -80,6 +80,7 @@ struct tp_handle {
   int num_tasks = 0;
   int ports_from_geometry = 0;
   int have_geometry = 0, have_tasks = 0, have_corr = 0, lpf_on = 0, planned = 0;
+  int map_valid = 0;  // d_tile_task belongs to the task list (tp_set_tile_ops writes both)
   int num_pairs = 0, corr_capacity = 0;
   int sched_tpb = 0, sched_nw = 0;  // fused-kernel schedule (0 = defaults)
   int clt_lpf_mask = 0;             // colours whose stored CLT carries the tp_set_lpf filter
@@ -117,14 +118,22 @@ static tp_status mark_work(tp_handle *h, cudaStream_t st) {
     h->err = std::string("event record: ") + cudaGetErrorString(e);
     return TP_ERR_CUDA;
   }
+  h->work_st = st;
   return TP_OK;
+}
+
+// orders st after the handle's work already enqueued (nothing to do where both are the handle's own
+// stream, which orders them itself)
+static cudaError_t wait_work(tp_handle *h, cudaStream_t st) {
+  if (st == h->stream && h->work_st == h->stream) return cudaSuccess;
+  return cudaStreamWaitEvent(st, h->ev_work, 0);
 }
 
 // A setter that overwrites a device buffer first waits for the handle's work in flight, which may
 // still read it on another stream: on the stream of its copy (after_work), or on the host before a
 // synchronous copy or a free (work_done).
 static tp_status after_work(tp_handle *h, cudaStream_t st, const char *where) {
-  CK(cudaStreamWaitEvent(st, h->ev_work, 0), where);
+  CK(wait_work(h, st), where);
   return TP_OK;
 }
 static tp_status work_done(tp_handle *h, const char *where) {
@@ -447,6 +456,7 @@ tp_status tp_create(const tp_config *cfg, tp_handle **out) {
   bool ok = cudaSetDevice(cfg->device) == cudaSuccess;
   ok = ok && cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) == cudaSuccess;
   ok = ok && cudaEventCreateWithFlags(&h->ev_work, cudaEventDisableTiming) == cudaSuccess;
+  h->work_st = h->stream;
   ok = ok && upload_kernel_constants() == cudaSuccess;
   ok = ok && upload_fused_constants() == cudaSuccess;
   ok = ok && upload_quad_constants() == cudaSuccess;
@@ -465,7 +475,8 @@ tp_status tp_create(const tp_config *cfg, tp_handle **out) {
   }
   ok = ok && dalloc(h, &h->d_task_txy, nt) == cudaSuccess && dalloc(h, &h->d_task_op, nt) == cudaSuccess;
   ok = ok && dalloc(h, &h->d_task_disp, nt) == cudaSuccess && dalloc(h, &h->d_task_xy, nt * S * 2) == cudaSuccess;
-  ok = ok && dalloc(h, &h->d_tile_op, nt) == cudaSuccess && dalloc(h, &h->d_tile_disp, nt) == cudaSuccess;
+  ok = ok && dalloc(h, &h->d_tile_op, 2 * nt) == cudaSuccess;  // tile ops, then disparities
+  if (ok) h->d_tile_disp = (float *)(h->d_tile_op + nt);
   ok = ok && dalloc(h, &h->d_num_tasks, 2 + nt / 1024 + 1) == cudaSuccess;  // count + per-block counts
   ok = ok && dalloc(h, &h->d_ports, nt * S * 2) == cudaSuccess;
   ok = ok && dalloc(h, &h->d_plan, nt * S * C) == cudaSuccess && dalloc(h, &h->d_tile_task, nt) == cudaSuccess;
@@ -501,7 +512,7 @@ tp_status tp_destroy(tp_handle *h) {
     dfree(h, h->d_kern[s]);
     dfree(h, h->d_kext[s]);
   }
-  void *bufs[] = {h->d_task_txy, h->d_task_op, h->d_task_disp, h->d_task_xy, h->d_tile_op, h->d_tile_disp,
+  void *bufs[] = {h->d_task_txy, h->d_task_op, h->d_task_disp, h->d_task_xy, h->d_tile_op,
                   h->d_num_tasks, h->d_ports, h->d_port_deriv, h->d_plan, h->d_tile_task, h->d_clt, h->d_corr,
                   h->d_disp, h->d_rbg, h->d_lpf_rbg, h->d_geom, h->d_rdist, h->d_corr_cfg,
                   h->d_tex, h->d_tex_aux, h->d_sens, h->d_dval, h->d_jac_e, h->d_jac_d, h->d_grad_d,
@@ -514,7 +525,6 @@ tp_status tp_destroy(tp_handle *h) {
     cudaEventDestroy(h->ev_stage);
   }
   if (h->h_stage_op) cudaFreeHost(h->h_stage_op);
-  if (h->h_stage_disp) cudaFreeHost(h->h_stage_disp);
   if (h->stream) cudaStreamDestroy(h->stream);
   if (h->ev_work) cudaEventDestroy(h->ev_work);
   delete h;
@@ -736,6 +746,15 @@ tp_status tp_set_color_scales(tp_handle *h, const float *scales) {
   return TP_OK;
 }
 
+// Rows without a gap go up as one piece: the copy engine moves a 2D copy at 60 GB/s, a plain one at
+// 210 GB/s (10 MB: 181 and 52 us).
+static cudaError_t upload_image(tp_handle *h, int cam, const void *image, size_t pitch, size_t es, cudaStream_t st) {
+  const size_t w = (size_t)h->cfg.width * es;
+  if (pitch == (size_t)h->cfg.width)
+    return cudaMemcpyAsync(h->d_images[cam], image, w * h->cfg.height, cudaMemcpyHostToDevice, st);
+  return cudaMemcpy2DAsync(h->d_images[cam], w, image, pitch * es, w, h->cfg.height, cudaMemcpyHostToDevice, st);
+}
+
 tp_status tp_set_image(tp_handle *h, int cam, const void *image, int dtype, size_t pitch) {
   if (h) h->images_since_fwd = 1;
   if (!h || !image) return TP_ERR_ARG;
@@ -745,9 +764,7 @@ tp_status tp_set_image(tp_handle *h, int cam, const void *image, int dtype, size
   if (pitch == 0) pitch = h->cfg.width;
   if (pitch < (size_t)h->cfg.width) return fail(h, TP_ERR_ARG, "tp_set_image: pitch < width");
   if (after_work(h, h->stream, "tp_set_image") != TP_OK) return TP_ERR_CUDA;
-  CK(cudaMemcpy2DAsync(h->d_images[cam], h->cfg.width * es, image, pitch * es, h->cfg.width * es, h->cfg.height,
-                       cudaMemcpyHostToDevice, h->stream),
-     "tp_set_image");
+  CK(upload_image(h, cam, image, pitch, es, h->stream), "tp_set_image");
   CK(cudaStreamSynchronize(h->stream), "tp_set_image");
   h->img_dtype[cam] = dtype;
   return TP_OK;
@@ -762,9 +779,7 @@ tp_status tp_set_image_async(tp_handle *h, int cam, const void *image, int dtype
   if (pitch == 0) pitch = h->cfg.width;
   if (pitch < (size_t)h->cfg.width) return fail(h, TP_ERR_ARG, "tp_set_image_async: pitch < width");
   if (after_work(h, pick_stream(h, stream), "tp_set_image_async") != TP_OK) return TP_ERR_CUDA;
-  CK(cudaMemcpy2DAsync(h->d_images[cam], h->cfg.width * es, image, pitch * es, h->cfg.width * es, h->cfg.height,
-                       cudaMemcpyHostToDevice, pick_stream(h, stream)),
-     "tp_set_image_async");
+  CK(upload_image(h, cam, image, pitch, es, pick_stream(h, stream)), "tp_set_image_async");
   h->img_dtype[cam] = dtype;
   return TP_OK;
 }
@@ -794,7 +809,7 @@ tp_status tp_set_tasks(tp_handle *h, const float *packed, int n) {
       xy[(size_t)i * 2 * S + k] = v;
     }
   }
-  CK(cudaStreamWaitEvent(h->stream, h->ev_work, 0), "tp_set_tasks");  // in-flight work reads the old list
+  CK(wait_work(h, h->stream), "tp_set_tasks");  // in-flight work reads the old list
   if (n > 0) {
     CK(cudaMemcpyAsync(h->d_task_txy, txy.data(), n * sizeof(int), cudaMemcpyHostToDevice, h->stream), "tp_set_tasks");
     CK(cudaMemcpyAsync(h->d_task_op, op.data(), n * sizeof(int), cudaMemcpyHostToDevice, h->stream), "tp_set_tasks");
@@ -803,6 +818,7 @@ tp_status tp_set_tasks(tp_handle *h, const float *packed, int n) {
   }
   CK(cudaStreamSynchronize(h->stream), "tp_set_tasks");
   h->num_tasks = n;
+  h->map_valid = 0;
   h->ports_from_geometry = 0;
   h->have_tasks = 1;
   h->planned = 0;
@@ -829,28 +845,26 @@ tp_status tp_set_tile_ops(tp_handle *h, const int *tile_op, const float *disp) {
     }
     n += tile_op[i] != 0;
   }
+  const size_t nt = h->ntiles;
   if (!h->h_stage_op) {
     if (cudaEventCreateWithFlags(&h->ev_stage, cudaEventDisableTiming) != cudaSuccess ||
-        cudaMallocHost((void **)&h->h_stage_op, h->ntiles * sizeof(int)) != cudaSuccess ||
-        cudaMallocHost((void **)&h->h_stage_disp, h->ntiles * sizeof(float)) != cudaSuccess) {
+        cudaMallocHost((void **)&h->h_stage_op, 2 * nt * sizeof(int)) != cudaSuccess) {
       cudaGetLastError();
       return fail(h, TP_ERR_NOMEM, "tp_set_tile_ops: staging buffers");
     }
   } else {
     CK(cudaEventSynchronize(h->ev_stage), "tp_set_tile_ops");  // the previous upload has read them
   }
-  memcpy(h->h_stage_op, tile_op, h->ntiles * sizeof(int));
-  memcpy(h->h_stage_disp, disp, h->ntiles * sizeof(float));
-  CK(cudaStreamWaitEvent(h->stream, h->ev_work, 0), "tp_set_tile_ops");
-  CK(cudaMemcpyAsync(h->d_tile_op, h->h_stage_op, h->ntiles * sizeof(int), cudaMemcpyHostToDevice, h->stream),
-     "tp_set_tile_ops");
-  CK(cudaMemcpyAsync(h->d_tile_disp, h->h_stage_disp, h->ntiles * sizeof(float), cudaMemcpyHostToDevice,
-                     h->stream),
+  memcpy(h->h_stage_op, tile_op, nt * sizeof(int));
+  memcpy(h->h_stage_op + nt, disp, nt * sizeof(float));
+  CK(wait_work(h, h->stream), "tp_set_tile_ops");
+  CK(cudaMemcpyAsync(h->d_tile_op, h->h_stage_op, 2 * nt * sizeof(int), cudaMemcpyHostToDevice, h->stream),
      "tp_set_tile_ops");
   CK(cudaEventRecord(h->ev_stage, h->stream), "tp_set_tile_ops");
   CK(launch_compact_tasks(h->d_tile_op, h->d_tile_disp, h->tilesX, h->ntiles, h->d_task_txy, h->d_task_op,
-                          h->d_task_disp, h->d_num_tasks, h->stream),
+                          h->d_task_disp, h->d_num_tasks, h->d_tile_task, h->stream),
      "tp_set_tile_ops");
+  h->map_valid = 1;
   h->num_tasks = n;
   h->ports_from_geometry = 1;
   h->have_tasks = 1;
@@ -1031,12 +1045,12 @@ static tp_status ensure_plan(tp_handle *h, cudaStream_t st) {
   if (!h->have_tasks) return fail(h, TP_ERR_STATE, "no tasks set (tp_set_tasks / tp_set_tile_ops)");
   if (h->ports_from_geometry && !h->have_geometry) return fail(h, TP_ERR_STATE, "geometry not set");
   if (h->planned) return TP_OK;
-  CK(cudaStreamWaitEvent(st, h->ev_work, 0), "plan");  // the task list, uploaded on the handle's stream
+  CK(wait_work(h, st), "plan");  // the task list, uploaded on the handle's stream
   SceneDev sc = scene_of(h);
   const bool with_deriv = h->adj_record && h->d_port_deriv && h->ports_from_geometry;
   if (with_deriv) sc.port_deriv = h->d_port_deriv;  // the adjoint's port derivatives, same ports
   CK(launch_plan(sc, st), "plan");
-  CK(launch_tile_task_map(sc, st), "tile map");
+  if (!h->map_valid) CK(launch_tile_task_map(sc, st), "tile map");
   h->planned = 1;
   h->deriv_valid = with_deriv ? 1 : 0;
   return TP_OK;
@@ -1212,7 +1226,7 @@ tp_status tp_get_num_tasks(const tp_handle *h, int *n) {
 static tp_status d2h(tp_handle *h, void *dst, const void *src, size_t bytes, const char *where) {
   if (!dst) return fail(h, TP_ERR_ARG, where);
   if (!src) return fail(h, TP_ERR_STATE, std::string(where) + ": not computed");
-  CK(cudaStreamWaitEvent(h->stream, h->ev_work, 0), where);
+  CK(wait_work(h, h->stream), where);
   CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->stream), where);
   CK(cudaStreamSynchronize(h->stream), where);
   return TP_OK;
@@ -1222,7 +1236,7 @@ static tp_status d2h(tp_handle *h, void *dst, const void *src, size_t bytes, con
 static tp_status d2h_async(tp_handle *h, void *dst, const void *src, size_t bytes, cudaStream_t st, const char *where) {
   if (!dst) return fail(h, TP_ERR_ARG, where);
   if (!src) return fail(h, TP_ERR_STATE, std::string(where) + ": not computed");
-  CK(cudaStreamWaitEvent(st, h->ev_work, 0), where);
+  CK(wait_work(h, st), where);
   CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st), where);
   return TP_OK;
 }
@@ -1331,7 +1345,7 @@ struct tp_batch {
 static std::vector<unsigned char> scene_key(tp_handle *h) {
   SceneDev sc = scene_of(h);
   sc.strips = nullptr;  // batched forwards do not record strip samples
-  const int sched[2] = {h->sched_tpb, h->sched_nw};
+  const int sched[3] = {h->sched_tpb, h->sched_nw, h->map_valid};
   std::vector<unsigned char> k(sizeof(SceneDev) + sizeof(CorrConst) + sizeof(sched));
   memcpy(k.data(), &sc, sizeof(SceneDev));
   memcpy(k.data() + sizeof(SceneDev), static_cast<const CorrConst *>(&h->corr_host), sizeof(CorrConst));
@@ -1419,6 +1433,7 @@ static tp_status batch_enqueue(tp_batch *b, int replan, cudaStream_t st) {
   if (need) {
     for (size_t i = 0; i < b->scenes.size(); i++) {
       const SceneDev &sc = b->h_scenes[i];
+      if (b->scenes[i]->map_valid) continue;  // written with the task list
       if (cudaMemsetAsync(sc.tile_task, 0xff, sizeof(int) * sc.tilesX * sc.tilesY, st) != cudaSuccess) {
         cudaGetLastError();
         return bfail(b, TP_ERR_CUDA, "batch: tile map");
@@ -1703,7 +1718,7 @@ tp_status tp_get_pair_maxima(tp_handle *h, float *out) {
     }
     h->pairmax_cap = need;
   }
-  CK(cudaStreamWaitEvent(h->stream, h->ev_work, 0), "tp_get_pair_maxima");
+  CK(wait_work(h, h->stream), "tp_get_pair_maxima");
   CK(launch_pair_maxima(scene_of(h), h->num_pairs, h->d_pairmax, h->stream), "tp_get_pair_maxima");
   if (mark_work(h, h->stream) != TP_OK) return TP_ERR_CUDA;
   return d2h(h, out, h->d_pairmax, need * sizeof(float), "tp_get_pair_maxima");
@@ -1752,8 +1767,8 @@ tp_status tp_rig_correlate(tp_handle *main_h, tp_handle *aux, float cm_max_norma
     }
     CK(cudaMemsetAsync(h->d_rig_corr, 0, (size_t)h->ntiles * TP_CORR * sizeof(float), st), "tp_rig_correlate");
   }
-  CK(cudaStreamWaitEvent(st, aux->ev_work, 0), "tp_rig_correlate");  // both cameras' forwards
-  CK(cudaStreamWaitEvent(st, h->ev_work, 0), "tp_rig_correlate");
+  CK(wait_work(aux, st), "tp_rig_correlate");  // both cameras' forwards
+  CK(wait_work(h, st), "tp_rig_correlate");
   const CorrConst cc = rig_corr_const(h);
   CK(launch_rig(scene_of(h), scene_of(aux), cc, h->d_rig_corr, h->d_rig_rec, cm_max_normalization, no_int_x0, st),
      "tp_rig_correlate");
@@ -1777,7 +1792,7 @@ tp_status tp_rig_lma(tp_handle *main_h, const tp_lma_params *p, int use_poly, in
     cudaGetLastError();
     return fail(h, TP_ERR_NOMEM, "tp_rig_lma: buffer");
   }
-  CK(cudaStreamWaitEvent(st, h->ev_work, 0), "tp_rig_lma");
+  CK(wait_work(h, st), "tp_rig_lma");
   CK(launch_rig_lma(scene_of(h), rig_corr_const(h), lma_const_of(prm), h->d_rig_corr, h->d_rig_rec, h->d_rig_tmp,
                     h->d_rig_tmp + (size_t)h->ntiles * TP_NDISP, use_poly, use_xy_poly, st),
      "tp_rig_lma");
@@ -1958,7 +1973,7 @@ tp_status tp_batch_process(tp_batch *b, int replan, void *stream) {
   cudaStream_t st = stream ? (cudaStream_t)stream : b->stream;
   for (tp_handle *h : b->scenes) {
     CK_B(cudaStreamSynchronize(h->stream));       // set-up copies on the handles' own streams
-    CK_B(cudaStreamWaitEvent(st, h->ev_work, 0));  // each scene's earlier work, on any stream
+    CK_B(wait_work(h, st));  // each scene's earlier work, on any stream
   }
   tp_status r = batch_tables(b);
   if (r != TP_OK) return r;
@@ -1996,7 +2011,7 @@ tp_status tp_batch_run_graph(tp_batch *b, void *stream) {
     b->graph_keys.clear();
     for (tp_handle *h : b->scenes) b->graph_keys.push_back(scene_key(h));
   }
-  for (tp_handle *h : b->scenes) CK_B(cudaStreamWaitEvent(st, h->ev_work, 0));
+  for (tp_handle *h : b->scenes) CK_B(wait_work(h, st));
   CK_B(cudaGraphLaunch(b->exec, st));
   CK_B(cudaEventRecord(b->ev_done, st));
   for (tp_handle *h : b->scenes)

@@ -161,7 +161,7 @@ cudaError_t launch_extract(const SceneDev &sc, cudaStream_t st);
 cudaError_t launch_imclt(const SceneDev &sc, cudaStream_t st);
 cudaError_t launch_imclt_fast(const SceneDev &sc, cudaStream_t st);
 cudaError_t launch_compact_tasks(const int *tile_op, const float *disparity, int tilesX, int num_tiles,
-                                 int *task_txy, int *task_op, float *task_disp, int *num_tasks_dev,
+                                 int *task_txy, int *task_op, float *task_disp, int *num_tasks_dev, int *tile_task,
                                  cudaStream_t st);
 cudaError_t upload_kernel_constants();
 // fused forward (tp_fused.cu): convert+correct, correlation, extraction in one kernel;

@@ -298,48 +298,6 @@ __global__ void tile_task_map_kernel(SceneDev sc) {
   }
 }
 
-// Row-major compaction of tiles with tile_op != 0 into the task list
-// (GPUTileProcessor.setFullFrameImages order).  One block; deterministic.
-__global__ void compact_tasks_kernel(const int *tile_op, const float *disparity, int tilesX, int num_tiles,
-                                     int *task_txy, int *task_op, float *task_disp, int *num_tasks) {
-  __shared__ int warp_sums[32];
-  __shared__ int base;
-  if (threadIdx.x == 0) base = 0;
-  __syncthreads();
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  for (int start = 0; start < num_tiles; start += blockDim.x) {
-    int i = start + threadIdx.x;
-    int op = (i < num_tiles) ? tile_op[i] : 0;
-    int flag = op != 0;
-    unsigned m = __ballot_sync(0xffffffffu, flag);
-    int pre = __popc(m & ((1u << lane) - 1u));
-    if (lane == 31) warp_sums[warp] = pre + flag;
-    __syncthreads();
-    if (warp == 0) {
-      int v = (lane < nwarps) ? warp_sums[lane] : 0;
-      int incl = v;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-      }
-      if (lane < nwarps) warp_sums[lane] = incl - v;
-    }
-    __syncthreads();
-    int pos = base + warp_sums[warp] + pre;
-    if (flag) {
-      int ty = i / tilesX, tx = i - ty * tilesX;
-      task_txy[pos] = tx | (ty << 16);
-      task_op[pos] = op;
-      task_disp[pos] = disparity ? disparity[i] : 0.0f;
-    }
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) base = pos + flag;
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *num_tasks = base;
-}
-
 // Sensors per thread: with few threads the kernel is a chain of dependent FP64 instructions, so each
 // takes one sensor; with many the FP64 pipes are full, and four sensors share the centre's part.
 // The line: about one warp per scheduler (32 x 4 x 152 threads).
@@ -369,37 +327,40 @@ cudaError_t launch_tile_task_map(const SceneDev &sc, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-// multi-block compaction: per-block counts, then each block adds the counts of
-// the blocks before it and scatters its tiles in row-major order
-constexpr int CB = 1024;
+// Row-major compaction of tiles with tile_op != 0 into the task list
+// (GPUTileProcessor.setFullFrameImages order), a block per 1024 tiles, deterministic: each block needs
+// the count of the tiles before its own.  Up to CB_SELF blocks it counts them itself (they are in L2, a
+// load per thread and block before it), so one launch does; beyond, a first launch counts per block.
+// tile_task (or null): the tile's task or -1.
+constexpr int CB = 1024, CB_SELF = 128;
+
 __global__ void compact_count_kernel(const int *tile_op, int num_tiles, int *block_counts) {
   const int i = blockIdx.x * CB + threadIdx.x;
   const int n = __syncthreads_count(i < num_tiles && tile_op[i] != 0);
   if (threadIdx.x == 0) block_counts[blockIdx.x] = n;
 }
 
-__global__ void compact_scatter_kernel(const int *tile_op, const float *disparity, int tilesX, int num_tiles,
-                                       const int *block_counts, int *task_txy, int *task_op, float *task_disp,
-                                       int *num_tasks) {
-  __shared__ int warp_sums[32];
+__global__ void __launch_bounds__(CB) compact_scatter_kernel(const int *tile_op, const float *disparity, int tilesX,
+                                                             int num_tiles, const int *block_counts, int *task_txy,
+                                                             int *task_op, float *task_disp, int *num_tasks,
+                                                             int *tile_task) {
+  __shared__ int warp_sums[32], before_sums[32];
   __shared__ int base;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (warp == 0) {
-    int b = 0;
-    for (int k = lane; k < blockIdx.x; k += 32) b += block_counts[k];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
-    if (lane == 0) {
-      base = b;
-      if (blockIdx.x == gridDim.x - 1) *num_tasks = b + block_counts[blockIdx.x];
-    }
+  int b = 0;  // tiles before this block's (this thread's share)
+  if (block_counts) {
+    for (int k = threadIdx.x; k < blockIdx.x; k += CB) b += block_counts[k];
+  } else {
+    for (int k = 0; k < blockIdx.x; k++) b += tile_op[k * CB + threadIdx.x] != 0;
   }
   const int i = blockIdx.x * CB + threadIdx.x;
   const int op = (i < num_tiles) ? tile_op[i] : 0;
   const int flag = op != 0;
   const unsigned m = __ballot_sync(0xffffffffu, flag);
   const int pre = __popc(m & ((1u << lane) - 1u));
+  b = __reduce_add_sync(0xffffffffu, b);
   if (lane == 31) warp_sums[warp] = pre + flag;
+  if (lane == 0) before_sums[warp] = b;
   __syncthreads();
   if (warp == 0) {
     const int v = warp_sums[lane];
@@ -409,32 +370,41 @@ __global__ void compact_scatter_kernel(const int *tile_op, const float *disparit
       const int t = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += t;
     }
+    const int before = __reduce_add_sync(0xffffffffu, before_sums[lane]);
+    if (lane == 31) {
+      base = before;
+      if (blockIdx.x == gridDim.x - 1) *num_tasks = before + incl;
+    }
     warp_sums[lane] = incl - v;
   }
   __syncthreads();
+  const int pos = base + warp_sums[warp] + pre;
   if (flag) {
-    const int pos = base + warp_sums[warp] + pre;
     const int ty = i / tilesX, tx = i - ty * tilesX;
     task_txy[pos] = tx | (ty << 16);
     task_op[pos] = op;
     task_disp[pos] = disparity ? disparity[i] : 0.0f;
   }
+  if (tile_task && i < num_tiles) tile_task[i] = flag ? pos : -1;
 }
 
-cudaError_t launch_compact_tasks(const int *tile_op, const float *disparity, int tilesX, int num_tiles,
-                                 int *task_txy, int *task_op, float *task_disp, int *num_tasks_dev,
-                                 cudaStream_t st) {
-  const int nb = (num_tiles + CB - 1) / CB;
-  if (nb <= 1) {
-    compact_tasks_kernel<<<1, 1024, 0, st>>>(tile_op, disparity, tilesX, num_tiles, task_txy, task_op, task_disp,
-                                             num_tasks_dev);
-    return cudaGetLastError();
-  }
-  int *counts = num_tasks_dev + 1;  // the caller sizes num_tasks_dev for 1 + nb ints
-  compact_count_kernel<<<nb, CB, 0, st>>>(tile_op, num_tiles, counts);
+static cudaError_t compact(const int *tile_op, const float *disparity, int tilesX, int num_tiles, int *task_txy,
+                           int *task_op, float *task_disp, int *num_tasks_dev, int *tile_task, int *counts,
+                           cudaStream_t st) {
+  const int nb = num_tiles > 0 ? (num_tiles + CB - 1) / CB : 1;
+  if (nb <= CB_SELF) counts = nullptr;
+  else compact_count_kernel<<<nb, CB, 0, st>>>(tile_op, num_tiles, counts);
   compact_scatter_kernel<<<nb, CB, 0, st>>>(tile_op, disparity, tilesX, num_tiles, counts, task_txy, task_op,
-                                            task_disp, num_tasks_dev);
+                                            task_disp, num_tasks_dev, tile_task);
   return cudaGetLastError();
+}
+
+// the caller sizes num_tasks_dev for 1 + number of 1024-tile blocks
+cudaError_t launch_compact_tasks(const int *tile_op, const float *disparity, int tilesX, int num_tiles,
+                                 int *task_txy, int *task_op, float *task_disp, int *num_tasks_dev, int *tile_task,
+                                 cudaStream_t st) {
+  return compact(tile_op, disparity, tilesX, num_tiles, task_txy, task_op, task_disp, num_tasks_dev, tile_task,
+                 num_tasks_dev + 1, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -456,15 +426,7 @@ cudaError_t compact_scratch_address(int **ptr) {
 cudaError_t launch_compact_tasks_scratch(const int *tile_op, const float *disparity, int tilesX, int num_tiles,
                                          int *task_txy, int *task_op, float *task_disp, int *num_tasks_dev,
                                          int *scratch, cudaStream_t st) {
-  const int nb = (num_tiles + CB - 1) / CB;
-  if (nb > COMPACT_SCRATCH_BLOCKS) return cudaErrorInvalidValue;
-  if (nb <= 1) {
-    compact_tasks_kernel<<<1, 1024, 0, st>>>(tile_op, disparity, tilesX, num_tiles, task_txy, task_op, task_disp,
-                                             num_tasks_dev);
-    return cudaGetLastError();
-  }
-  compact_count_kernel<<<nb, CB, 0, st>>>(tile_op, num_tiles, scratch);
-  compact_scatter_kernel<<<nb, CB, 0, st>>>(tile_op, disparity, tilesX, num_tiles, scratch, task_txy, task_op,
-                                            task_disp, num_tasks_dev);
-  return cudaGetLastError();
+  if ((num_tiles + CB - 1) / CB > COMPACT_SCRATCH_BLOCKS) return cudaErrorInvalidValue;
+  return compact(tile_op, disparity, tilesX, num_tiles, task_txy, task_op, task_disp, num_tasks_dev, nullptr, scratch,
+                 st);
 }

@@ -86,3 +86,78 @@ def test_corner_rounding_of_given_ports(step):
     want = np.where(t > hi, hi - ((hi % 2) != par), np.where(t < lo, lo + ((lo % 2) != par), t))
     assert np.array_equal(tl[:, :, 0], want.astype(int))
     assert np.array_equal(res[:, :, 0], (-(p - t)).astype(np.float32))
+
+
+@pytest.mark.parametrize("n", [1, 31, 1024, 1025, 128 * 1024, 128 * 1024 + 1, 300001])
+def test_compaction_sizes(n):
+    """One block, block edges, the largest list whose blocks count for themselves and the first beyond."""
+    import ctypes as C
+    torch = pytest.importorskip("torch")
+    from tileproc import _lib as L
+    lib = L.load()
+    rng = np.random.default_rng(n)
+    op = np.where(rng.random(n) < 0.3, rng.integers(1, 99, n), 0).astype(np.int32)
+    op[-1] = 7
+    d = rng.random(n).astype(np.float32)
+    dop, dd = torch.from_numpy(op).cuda(), torch.from_numpy(d).cuda()
+    out = torch.zeros((3, n), dtype=torch.int32, device="cuda")
+    num = torch.zeros(1, dtype=torch.int32, device="cuda")
+    p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
+    assert lib.tp_compact_tile_ops_noalloc(p(dop), p(dd), 640, n, p(out[0]), p(out[1]), p(out[2]), p(num), None) == L.TP_OK
+    torch.cuda.synchronize()
+    i = np.nonzero(op)[0]
+    k = int(num.item())
+    assert k == len(i)
+    got = out[:, :k].cpu().numpy()
+    assert np.array_equal(got[0], (i % 640) | ((i // 640) << 16))
+    assert np.array_equal(got[1], op[i]) and np.array_equal(got[2].view(np.float32), d[i])
+
+
+def test_tile_map_follows_the_task_list():
+    """IMCLT reads the tile -> task map: sparse tile ops, then packed tasks, then tile ops again, against
+    handles that saw only one list."""
+    from tileproc import synth
+    sc = synth.make_scene("quad_mono", seed=5, width=128, height=96)
+    T = 16 * 12
+    rng = np.random.default_rng(3)
+    ops = [(rng.random(T) < f).astype(np.int32) for f in (0.5, 0.7)]
+    i = np.nonzero(rng.random(T) < 0.4)[0]
+    with make_gpu(sc) as tp:
+        tp.setFullFrameImages(2.0)
+        tp.execPorts()
+        xy = tp.getPorts()[i].astype(np.float32)
+        packed = tp.packTasks(np.ones(len(i)), i % 16, i // 16, xy)
+
+    def frame(tp, step):
+        if step == 1:
+            tp.setTasks(packed)
+        else:
+            tp.setFullFrameImages(2.0, tile_op=ops[step // 2])
+        tp.execConverCorrectTiles()
+        tp.execImcltRbg()
+        return tp.getRBG(1)
+    with make_gpu(sc) as tp:
+        got = [frame(tp, k) for k in range(3)]
+    for k in range(3):
+        with make_gpu(sc) as tp:
+            assert np.array_equal(got[k], frame(tp, k))
+
+
+def test_padded_and_packed_images():
+    from tileproc import GPUTileProcessor, synth
+    import ctypes as C
+    from tileproc import _lib as L
+    sc = synth.make_scene("quad_mono", seed=6, width=64, height=48)
+    res = []
+    for pad in (0, 24):
+        with GPUTileProcessor(4, 64, 48) as tp:
+            tp.setGeometry(sc["geometry"])
+            for s in range(4):
+                a = np.full((48, 64 + pad), np.nan, np.float32)
+                a[:, :64] = sc["images"][s]
+                tp._ck(tp._lib.tp_set_image(tp.h, s, C.c_void_p(a.ctypes.data), L.TP_F32, 64 + pad), "tp_set_image")
+            tp.setCorrelation()
+            tp.setFullFrameImages(3.0)
+            tp.process()
+            res.append((tp.getClt(), tp.getDisparity()))
+    assert np.array_equal(res[0][0], res[1][0]) and np.array_equal(res[0][1], res[1][1], equal_nan=True)
