@@ -461,6 +461,7 @@ tp_status tp_create(const tp_config *cfg, tp_handle **out) {
   ok = ok && upload_fused_constants() == cudaSuccess;
   ok = ok && upload_quad_constants() == cudaSuccess;
   ok = ok && upload_many_constants() == cudaSuccess;
+  ok = ok && upload_adjoint_many_constants() == cudaSuccess;
   ok = ok && upload_texture_constants() == cudaSuccess;
   ok = ok && upload_adjoint_constants() == cudaSuccess;
   ok = ok && upload_kernprep_constants() == cudaSuccess;
@@ -991,31 +992,48 @@ tp_status tp_set_corr(tp_handle *h, const tp_corr_params *p, const tp_pair *pair
       }
       cd.gen_cell[i][e] = cells;
     }
-  // the adjoint's rounds: greedily, in pair order, up to 4 combined-strip pairs on distinct sensors
-  {
+  // a lane's place among the lanes before it in its strip row that fall into the same cell, per side
+  // (bits 18-21, 22-25), and the pair's largest such place (bits 26-29)
+  for (int i = 0; i < np; i++) {
+    int most = 0;
+    for (int e = 0; e < 32; e++)
+      for (int side = 0; side < 2; side++) {
+        if ((cd.gen_cell[i][e] >> (16 + side)) & 1) continue;
+        int place = 0;
+        for (int f = e - e % 15; f < e; f++)
+          place += !((cd.gen_cell[i][f] >> (16 + side)) & 1) &&
+                   ((cd.gen_cell[i][f] ^ cd.gen_cell[i][e]) >> (8 * side) & 255) == 0;
+        cd.gen_cell[i][e] |= place << (18 + 4 * side);
+        if (e < 30 && place > most) most = place;
+      }
+    for (int e = 0; e < 32; e++) cd.gen_cell[i][e] |= most << 26;
+  }
+  // the adjoint's rounds: greedily, in pair order, up to 4 (8) combined-strip pairs on distinct sensors
+  auto schedule = [&](short *rounds, int width) {
     std::vector<int> left;
     for (int i = 0; i < np; i++)
       if (pairs[i].in_combo) left.push_back(i);
     int nr = 0;
-    while (!left.empty()) {
+    for (; !left.empty(); nr++) {
       std::vector<int> rest;
       unsigned long long used = 0;
       int k = 0;
       for (int i : left) {
         const unsigned long long m = (1ull << pairs[i].cam1) | (1ull << pairs[i].cam2);
-        if (k < 4 && !(used & m)) {
-          cd.adj_round[nr][k++] = (short)i;
+        if (k < width && !(used & m)) {
+          rounds[nr * width + k++] = (short)i;
           used |= m;
         } else {
           rest.push_back(i);
         }
       }
-      for (; k < 4; k++) cd.adj_round[nr][k] = -1;
-      nr++;
+      for (; k < width; k++) rounds[nr * width + k] = -1;
       left.swap(rest);
     }
-    cd.adj_rounds = nr;
-  }
+    return nr;
+  };
+  cd.adj_rounds = schedule(&cd.adj_round[0][0], 4);
+  cd.adj_rounds8 = schedule(&cd.adj_round8[0][0], 8);
   if (work_done(h, "tp_set_corr") != TP_OK) return TP_ERR_CUDA;  // before the free and the table copy
   if (np > h->corr_capacity) {
     dfree(h, h->d_corr);

@@ -87,9 +87,14 @@ struct CorrDev : CorrConst {
   // sensors are all distinct, so the four warps of a tile add their pairs' CLT gradients into
   // disjoint sensors, and every sensor's gradient is summed in the same pair order in every run
   short adj_round[TP_MAXP][4];
+  // the same with up to 8 pairs a round, two a warp (the many-pair adjoint)
+  short adj_round8[TP_MAXP][8];
+  int adj_rounds8;
   // strip taps of general pairs (kind 4) for the first 32 strip entries: the bilinear fractions of the two
   // sides (x, y below; x, y above) and the cells, 8 bits a side, bit 16 / 17 set where a side falls
-  // outside the surface.  They are the same for every tile.
+  // outside the surface; then, for adding into the cells without conflicts, the lane's place among its
+  // row's lanes of the same cell (4 bits a side) and the pair's largest place.  They are the same for
+  // every tile.
   alignas(16) float gen_tap[TP_MAXP][32][4];
   int gen_cell[TP_MAXP][32];
 };
@@ -204,6 +209,10 @@ cudaError_t launch_compact_tasks_scratch(const int *tile_op, const float *dispar
 // adjoint (tp_adjoint.cu): per-tile dd/dport, Jacobian rows, loss gradient
 cudaError_t upload_adjoint_constants();
 int adjoint_smem_bytes(int S, int C);
+// its per-tile kernel for mono scenes with many general pairs and recorded strips (tp_adjoint_many.cu)
+cudaError_t upload_adjoint_many_constants();
+bool adjoint_many_ok(const SceneDev &sc, int recompute);
+cudaError_t launch_adjoint_many(const SceneDev &sc, const CorrConst &cc, float *sens, float *dval, cudaStream_t st);
 cudaError_t launch_adjoint(const SceneDev &sc, const CorrConst &cc, int recompute, int use_strips, float *sens, float *dval,
                            const float *dl_dd, float *jac_e, float *jac_d, float *grad_d, float *partial,
                            float *grad_e, cudaStream_t st);
