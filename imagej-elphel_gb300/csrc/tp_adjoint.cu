@@ -417,6 +417,8 @@ cudaError_t launch_adjoint(const SceneDev &sc, const CorrConst &cc, int recomput
   cudaError_t e;
   if (as.use_strips && adjoint_many_ok(sc, recompute)) {
     e = launch_adjoint_many(sc, cc, sens, dval, st);
+  } else if (as.use_strips && adjoint_quad_ok(sc, recompute)) {
+    e = launch_adjoint_quad(sc, cc, sens, dval, st);
   } else {
     int res = 0;
     e = kernel_residency((const void *)adjoint_kernel, 32 * AD_NW, bytes, &res);

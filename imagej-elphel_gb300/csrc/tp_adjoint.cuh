@@ -5,6 +5,12 @@
 
 namespace {
 
+// a compile-time index as a type
+template <int N>
+struct Int {
+  static constexpr int value = N;
+};
+
 constexpr float K16 = 0.19634954084936207f;  // pi / 16
 
 struct AdjShape {
@@ -173,26 +179,15 @@ __device__ __forceinline__ float strip_entry(const float *c, const short *strip_
 
 constexpr int AD_NW = 4;  // warps per tile
 
-// dd/d(port x, port y) of one (sensor, colour) sub-tile, 8-lane group (lane r holds row r):
-// the dd/dCLT gl of the sub-tile is taken back once through the phase rotation, the kernel
-// convolution and the 2D DCT-IV/DST-IV (symmetric transforms: the transpose runs through the same
-// butterflies) to the folded tile, which is dotted with the fold of the pixels under the
-// derivative window, one fold per direction, plus the rotation's own derivative.  gl is
-// overwritten (with the folded gradient) where `own` is set.  Result in out[] of every lane.
-// ASYNC: w is a staged window whose copies are waited for before it is read; tbq may lie over clt.
-template <bool ASYNC = false, typename PIX>
-__device__ __forceinline__ void shift_sens(const SceneDev &sc, const PIX &w, const SubtilePlan &p, int s,
-                                           const float *clt, float *gl_all, float *tbq, int r, bool own,
-                                           float out[2]) {
-  const float *kp = (p.kidx >= 0) ? sc.kernels[s] + (size_t)p.kidx * TP_CLT : nullptr;
-  float ahs, ahc, avs, avc;
-  __sincosf(CUDART_PI_F * 0.0625f * p.rx, &ahs, &ahc);
-  __sincosf(CUDART_PI_F * 0.0625f * p.ry, &avs, &avc);
-  const FoldIdx fv = fold_idx(r);
+// First part of a sub-tile's sensitivity to its residual shift, 8-lane group (lane r holds row r): the
+// rotation's own derivative dotted with the dd/dCLT gl (gdir, this lane's part), and gl taken back through the
+// phase rotation, the kernel convolution and the 2D DCT-IV/DST-IV (symmetric transforms: the transpose runs
+// through the same butterflies) to the folded tile (gf, row r).  tbq may lie over clt.
+__device__ __forceinline__ void shift_grad(const SubtilePlan &p, const float *kp, const float *clt, const float *gl, float *tbq,
+                                           int r, float gdir[2], float gf[4][8]) {
   // the rotation's own derivative (pi/16 (2k+1) x the CLT turned by 90 degrees) dotted with dd/dCLT
-  float gdir[2] = {0.f, 0.f};
-  float gf[4][8];
-  load_rows(gl_all, r, gf);
+  gdir[0] = gdir[1] = 0.f;
+  load_rows(gl, r, gf);
 #pragma unroll
   for (int w4 = 0; w4 < 2; w4++) {
     float4 c4[4];
@@ -209,8 +204,7 @@ __device__ __forceinline__ void shift_sens(const SceneDev &sc, const PIX &w, con
       gdir[1] = fmaf(fy, (g2 * c0 - g0 * c2) + (g3 * c1 - g1 * c3), gdir[1]);
     }
   }
-  float *gfs = gl_all + r * 8;  // gfs[m * 64 + j] for folded row r
-  if (ASYNC) __syncwarp();  // the CLT is read
+  __syncwarp();  // the CLT is read
   rotate_t(gf, p.rx, p.ry, r);
   convolve_t(gf, kp, r);
 #pragma unroll
@@ -220,11 +214,52 @@ __device__ __forceinline__ void shift_sens(const SceneDev &sc, const PIX &w, con
     group_transpose(u, tbq, r);
     dtt4_fast(u, gf[m], m & 1);
   }
-  if (own) {
+}
+
+// Last part: the lanes' parts summed, then dd/d(port x, port y) in every lane.
+// residual = TL - px: dd/dpx = -dd/drx; the kernel-centre offsets add the dependence of px, py
+// on the port through kdx, kdy (ImageDtt.java:4930-4939)
+__device__ __forceinline__ void shift_out(const SceneDev &sc, const SubtilePlan &p, int s, float gdir[2], float out[2]) {
 #pragma unroll
-    for (int m = 0; m < 4; m++) {
-      *(float4 *)(gfs + m * 64) = make_float4(gf[m][0], gf[m][1], gf[m][2], gf[m][3]);
-      *(float4 *)(gfs + m * 64 + 4) = make_float4(gf[m][4], gf[m][5], gf[m][6], gf[m][7]);
+  for (int dir = 0; dir < 2; dir++) {
+    gdir[dir] += __shfl_xor_sync(0xffffffffu, gdir[dir], 1);
+    gdir[dir] += __shfl_xor_sync(0xffffffffu, gdir[dir], 2);
+    gdir[dir] += __shfl_xor_sync(0xffffffffu, gdir[dir], 4);
+  }
+  const float gpx = -gdir[0], gpy = -gdir[1];
+  out[0] = gpx;
+  out[1] = gpy;
+  if (p.kidx >= 0) {
+    const float4 e1 = __ldg((const float4 *)(sc.kext[s] + (size_t)p.kidx * 8) + 1);
+    out[0] = gpx * (1.0f - e1.x) - gpy * e1.z;
+    out[1] = -gpx * e1.y + gpy * (1.0f - e1.w);
+  }
+}
+
+// dd/d(port x, port y) of one (sensor, colour) sub-tile, 8-lane group: its dd/dCLT gl taken back to the folded
+// tile, which is dotted with the fold of the pixels under the derivative window, one fold per direction,
+// plus the rotation's own derivative.  gl is overwritten (with the folded gradient) where `own` is set.
+// ASYNC: w is a staged window whose copies are waited for before it is read.
+template <bool ASYNC = false, typename PIX>
+__device__ __forceinline__ void shift_sens(const SceneDev &sc, const PIX &w, const SubtilePlan &p, int s,
+                                           const float *clt, float *gl_all, float *tbq, int r, bool own,
+                                           float out[2]) {
+  const float *kp = (p.kidx >= 0) ? sc.kernels[s] + (size_t)p.kidx * TP_CLT : nullptr;
+  float ahs, ahc, avs, avc;
+  __sincosf(CUDART_PI_F * 0.0625f * p.rx, &ahs, &ahc);
+  __sincosf(CUDART_PI_F * 0.0625f * p.ry, &avs, &avc);
+  const FoldIdx fv = fold_idx(r);
+  float gdir[2];
+  float *gfs = gl_all + r * 8;  // gfs[m * 64 + j] for folded row r
+  {
+    float gf[4][8];
+    shift_grad(p, kp, clt, gl_all, tbq, r, gdir, gf);
+    if (own) {
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        *(float4 *)(gfs + m * 64) = make_float4(gf[m][0], gf[m][1], gf[m][2], gf[m][3]);
+        *(float4 *)(gfs + m * 64 + 4) = make_float4(gf[m][4], gf[m][5], gf[m][6], gf[m][7]);
+      }
     }
   }
   if (ASYNC) cp_async_wait_all();
@@ -264,22 +299,7 @@ __device__ __forceinline__ void shift_sens(const SceneDev &sc, const PIX &w, con
     }
     gdir[dir] += acc;
   }
-#pragma unroll
-  for (int dir = 0; dir < 2; dir++) {
-    gdir[dir] += __shfl_xor_sync(0xffffffffu, gdir[dir], 1);
-    gdir[dir] += __shfl_xor_sync(0xffffffffu, gdir[dir], 2);
-    gdir[dir] += __shfl_xor_sync(0xffffffffu, gdir[dir], 4);
-  }
-  // residual = TL - px: dd/dpx = -dd/drx; the kernel-centre offsets add the dependence of px, py
-  // on the port through kdx, kdy (ImageDtt.java:4930-4939)
-  const float gpx = -gdir[0], gpy = -gdir[1];
-  out[0] = gpx;
-  out[1] = gpy;
-  if (p.kidx >= 0) {
-    const float4 e1 = __ldg((const float4 *)(sc.kext[s] + (size_t)p.kidx * 8) + 1);
-    out[0] = gpx * (1.0f - e1.x) - gpy * e1.z;
-    out[1] = -gpx * e1.y + gpy * (1.0f - e1.w);
-  }
+  shift_out(sc, p, s, gdir, out);
 }
 
 // x = T^T y for the DCT-IIe / DST-IIe of dtt2e_fast (its transposed data flow)

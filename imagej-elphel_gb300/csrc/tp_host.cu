@@ -462,6 +462,7 @@ tp_status tp_create(const tp_config *cfg, tp_handle **out) {
   ok = ok && upload_quad_constants() == cudaSuccess;
   ok = ok && upload_many_constants() == cudaSuccess;
   ok = ok && upload_adjoint_many_constants() == cudaSuccess;
+  ok = ok && upload_adjoint_quad_constants() == cudaSuccess;
   ok = ok && upload_texture_constants() == cudaSuccess;
   ok = ok && upload_adjoint_constants() == cudaSuccess;
   ok = ok && upload_kernprep_constants() == cudaSuccess;

@@ -57,3 +57,53 @@ def test_many_pair_adjoint_matches_general(S, w, h, u16, kern, fill, drop, shrin
     assert np.all(np.abs(s0 - s1) <= 2e-5 * np.maximum(scale, 1e-6))
     for x, y in zip(b[:3], c[:3]):  # and it repeats exactly
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("dark,w,h,u16,kern,fill,drop,flat,corr_kw", [
+    (True, 72, 56, True, True, 1.0, (), False, {}),
+    (False, 16, 16, True, False, 1.0, (), False, {}),
+    (False, 72, 56, True, True, 1.0, (), True, {}),
+    (False, 56, 72, False, True, 0.5, (0,), False, {}),
+    (False, 104, 40, True, True, 1.0, (2, 5), False, {"corr_wndy_size": 1}),
+    (False, 40, 40, False, False, 1.0, (1, 0), True, {}),
+])
+def test_bayer_quad_adjoint_matches_general(dark, w, h, u16, kern, fill, drop, flat, corr_kw):
+    """The Bayer quad kernel (tp_adjoint_quad.cu) the same way: pairs and whole couples left out of the
+    combination, a one-row strip, tiles without a peak, both image types, sparse tasks."""
+    from helpers import make_gpu
+    from test_gpu_quad import PAIRS
+    sc = synth.make_scene("quad_bayer", seed=91, width=w, height=h)
+    if flat:
+        sc["images"][:, :, : w // 2] = 2048
+    if dark:  # windows of zeros: no correlation, no peak
+        sc["images"][:, :, : w // 2] = 0
+    if not u16:
+        sc["images"] = sc["images"].astype(np.float32)
+    rng = np.random.default_rng(w)
+    for k in ("azimuth", "tilt", "roll", "zoom"):
+        sc["geometry"][k] = (2e-4 * rng.standard_normal(4)).tolist()
+    pairs = [list(p) for p in PAIRS]
+    for i in drop:
+        pairs[i][3] = 0
+    T = (w // 8) * (h // 8)
+    op = (rng.uniform(size=T) < fill).astype(np.int32)
+    op[0] = op[-1] = 1
+    kernels = synth.random_clt_kernels(rng, 4, h // 16 + 2, w // 16 + 2, 3, strength=0.05) if kern else (None, None)
+    got = []
+    with make_gpu(sc, *kernels) as tp:
+        tp.setCorrelation(pairs=pairs, **corr_kw)
+        tp.setFullFrameImages(sc["disparity_gt"].reshape(-1).astype(np.float32), tile_op=op)
+        for _ in range(3):
+            tp.process()
+            tp.backward()
+            got.append((tp.getPortSensitivities()[op != 0], tp.getDisparityJacobian()[2][op != 0]))
+    (s0, d0), (s1, d1), (s2, d2) = got
+    np.testing.assert_array_equal(d0, d1)
+    assert np.isfinite(d0).any()
+    if dark:
+        assert np.isnan(d0).any()
+    # the same sums in another order, as above
+    scale = np.abs(s0).reshape(len(s0), -1).max(1)[:, None, None]
+    assert np.all(np.abs(s0 - s1) <= 2e-5 * np.maximum(scale, 1e-6))
+    np.testing.assert_array_equal(s1, s2)
+    np.testing.assert_array_equal(d1, d2)
