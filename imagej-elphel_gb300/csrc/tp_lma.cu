@@ -13,21 +13,34 @@
 //    group (s = sqrt 2 for the diagonal group) with Levenberg-Marquardt and
 //    the reference's lambda schedule (Correlations2dLMA.java:211-640).
 //
-// One warp per tile: cells and samples are spread over the lanes, the region
+// One warp per fit: cells and samples are spread over the lanes, the region
 // growth runs one step per warp-synchronous pass, and the normal equations are
-// reduced across the warp and solved redundantly by every lane (FP32).
+// reduced across the warp and solved redundantly by every lane (FP32).  The
+// main fits are one launch, the four orientation fits of a tile another.
 #include "tp_dtt.cuh"
 
 #include <cmath>
 
 namespace {
 
-constexpr int LMA_NW = 4;             // warps (tiles) per CTA
+constexpr int LMA_NW = 2;             // warps (tiles) per CTA
+// packed normal equations of n parameters: A (upper n x n), b (n), weighted rms^2
+__host__ __device__ constexpr int lma_neq(int n) { return n * (n + 1) / 2 + n + 1; }
+constexpr int LMA_RED = 36;           // row stride of the reduction buffer: 16-byte reads by 28 lanes without bank conflicts
 constexpr int LMA_ORTHO_ENTRIES = 81;  // addSamples enumeration, ortho group
 constexpr int LMA_DIAG_ENTRIES = 145;  // addSamples enumeration, diagonal group
 constexpr int LMA_MAX_SAMPLES = 162;   // 9x9 window cells per group
 constexpr int LMA_NP = 6;              // X0, WM, WYD, WXY, AG0, AG1
-constexpr int LMA_STAGE_PAIRS = 6;     // pair surfaces staged in shared memory (the quad layout's six)
+
+// The parameters a fit solves for.  What is held by construction is left out (the solution is the same, its row of
+// the system is the identity): WYD unless adjust_wy is set, AG1 when all pairs are of one group.
+template <bool WY, bool TWO>
+struct LmaPar {
+  static constexpr int wxy = WY ? 3 : 2, ag = wxy + 1, n = ag + 1 + TWO;
+  static constexpr int na = n * (n + 1) / 2;                                     // packed upper triangle
+  static constexpr int wxy2 = wxy * n - wxy * (wxy - 1) / 2;                     // its (wxy, wxy) entry; (1, 1) is n
+};
+constexpr int LMA_DIRS = 4;            // orientation fits of a tile, a warp each
 constexpr int LMA_POLY_CHUNK = 6;      // pairs per polynomial-mismatch pass (one solving lane each)
 constexpr int LMA_POLY_SCRATCH = 48;   // doubles of solver scratch per lane
 
@@ -36,27 +49,17 @@ constexpr int LMA_POLY_SCRATCH = 48;   // doubles of solver scratch per lane
 __device__ signed char g_lma_cx[LMA_ORTHO_ENTRIES + LMA_DIAG_ENTRIES];
 __device__ signed char g_lma_cy[LMA_ORTHO_ENTRIES + LMA_DIAG_ENTRIES];
 
-__device__ __forceinline__ void cp_async4(float *dst_smem, const float *src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(float *dst_smem, const float *src) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-}
-
 // per-warp shared memory (floats): group surfaces [2][225], samples x/y/v/w [4][162] + group bytes,
-// the reduction buffer [28][33], accepted / trial normal equations, and the staged pair surfaces,
-// which start on a 16-byte boundary for the 8-byte asynchronous copies
-constexpr int LMA_OFF_RED = 450 + 4 * LMA_MAX_SAMPLES + LMA_MAX_SAMPLES / 4 + 1;
-constexpr int LMA_OFF_STAGE = ((LMA_OFF_RED + 28 * 33 + 64) + 3) & ~3;
-constexpr int LMA_OFF_RES = LMA_OFF_STAGE + LMA_STAGE_PAIRS * 225;  // [4][4] orientation fits
-constexpr int LMA_PER_WARP = ((LMA_OFF_RES + 16) + 3) & ~3;
-static_assert(LMA_OFF_STAGE % 4 == 0 && LMA_PER_WARP % 4 == 0, "staged surfaces must be 16-byte aligned");
+// the reduction buffer [28][36], accepted / trial normal equations.  The pair surfaces are read from
+// global memory for each fit's group sums.
+constexpr int LMA_OFF_RED = (450 + 4 * LMA_MAX_SAMPLES + LMA_MAX_SAMPLES / 4 + 1 + 3) & ~3;
+constexpr int LMA_PER_WARP = LMA_OFF_RED + lma_neq(LMA_NP) * LMA_RED + 64;
+static_assert(LMA_PER_WARP % 4 == 0, "16-byte rows in the reduction buffer");
 // polynomial mismatch scratch: moments over the reduction buffer, solver rows over the group
-// surfaces and samples, both 8-byte aligned and clear of the staged surfaces
-static_assert(((LMA_OFF_RED + 1) & ~1) + 2 * 21 * LMA_POLY_CHUNK <= LMA_OFF_STAGE, "moments overlap the stage");
+// surfaces and samples, both 8-byte aligned
+static_assert(((LMA_OFF_RED + 1) & ~1) + 2 * 21 * LMA_POLY_CHUNK <= LMA_PER_WARP, "moments past the warp's memory");
 static_assert(2 * LMA_POLY_SCRATCH * LMA_POLY_CHUNK <= LMA_OFF_RED, "solver scratch overlaps the moments");
+static_assert(4 * LMA_DIRS * LMA_PER_WARP + 128 <= 48 << 10, "within the default shared memory limit");
 static_assert(LMA_POLY_CHUNK <= 32, "one solving lane per pair");
 
 struct LmaDev {
@@ -155,62 +158,75 @@ __device__ __forceinline__ unsigned bit_range(int a, int b) {
   return (b < a) ? 0u : (((2u << b) - 1u) & ~((1u << a) - 1u));
 }
 
-constexpr int LMA_NEQ = 28;  // packed normal equations: A (upper 6x6, 21), b (6), weighted rms^2
-// floats from the sample arrays to the end of the reduction buffer, free before the samples exist
 
-// Weighted normal equations of the samples at parameters av (getFxJt, getWJtJlambda, getWYmFxRms),
-// written to out[LMA_NEQ] for every lane: per-lane partial sums are transposed through red
-// [LMA_NEQ][33] and lane k sums row k in a fixed order.
+// Weighted normal equations of the samples at parameters av (getFxJt, getWJtJlambda, getWYmFxRms), packed into
+// out (A upper NP x NP, b, weighted rms^2) for every lane: per-lane partial sums are transposed through red
+// [lma_neq(NP)][LMA_RED] and lane k sums row k in lane order (lanes past the sample count hold zeros, so the sum
+// ends at the last group of four that holds a sample).
+template <bool WY, bool TWO>
 __device__ __forceinline__ void lma_eval(const float *sx, const float *sy, const float *sv, const float *sw,
-                                         const unsigned char *sg, int gdiag_bits, int ns, const float av[LMA_NP],
+                                         const unsigned char *sg, int gdiag_bits, int ns,
+                                         const float av[LmaPar<WY, TWO>::n],
                                          float w_wm, float w_wxy, float half_width, float *red, float *out,
                                          int lane) {
-  float A[21], b[LMA_NP], r2 = 0.f;
+  using Par = LmaPar<WY, TWO>;
+  constexpr int NP = Par::n, NA = Par::na;
+  float A[NA], b[NP], r2 = 0.f;
 #pragma unroll
-  for (int k = 0; k < 21; k++) A[k] = 0.f;
+  for (int k = 0; k < NA; k++) A[k] = 0.f;
 #pragma unroll
-  for (int k = 0; k < LMA_NP; k++) b[k] = 0.f;
-  const float Wy = av[1] + av[2], Wx = Wy + av[3];
+  for (int k = 0; k < NP; k++) b[k] = 0.f;
+  const float Wy = WY ? av[1] + av[2] : av[1], Wx = Wy + av[Par::wxy];
   const float iWx = 1.0f / Wx, iWy = 1.0f / Wy;
   for (int n = lane; n < ns; n += 32) {
-    const int g = sg[n];
+    const int g = TWO ? sg[n] : 0;
     const float ws = ((gdiag_bits >> g) & 1) ? 1.41421356237f : 1.0f;
-    const float Ag = g ? av[5] : av[4];
+    const float Ag = g ? av[NP - 1] : av[Par::ag];
     const float dxw = ws * (sx[n] - av[0]) * iWx, dyw = ws * sy[n] * iWy;
     const float d = 1.0f - dxw * dxw - dyw * dyw;
     const float e = sv[n] - d * Ag, w = sw[n], wr = w * e;
     const float dfdWx = 2.0f * Ag * dxw * dxw * iWx, dfdWy = 2.0f * Ag * dyw * dyw * iWy;
-    const float j[LMA_NP] = {2.0f * ws * Ag * dxw * iWx, dfdWx + dfdWy, dfdWx + dfdWy, dfdWx,
-                             (g == 0) ? d : 0.0f, (g == 1) ? d : 0.0f};
+    float j[NP];
+    j[0] = 2.0f * ws * Ag * dxw * iWx;
+    j[1] = dfdWx + dfdWy;
+    if (WY) j[2] = j[1];
+    j[Par::wxy] = dfdWx;
+    j[Par::ag] = (g == 0) ? d : 0.0f;
+    if (TWO) j[NP - 1] = (g == 1) ? d : 0.0f;
     r2 = fmaf(wr, e, r2);
     int k = 0;
 #pragma unroll
-    for (int a = 0; a < LMA_NP; a++) {
+    for (int a = 0; a < NP; a++) {
       b[a] = fmaf(j[a], wr, b[a]);
       const float wj = w * j[a];
 #pragma unroll
-      for (int c = a; c < LMA_NP; c++) {
+      for (int c = a; c < NP; c++) {
         A[k] = fmaf(wj, j[c], A[k]);
         k++;
       }
     }
   }
 #pragma unroll
-  for (int k = 0; k < 21; k++) red[k * 33 + lane] = A[k];
+  for (int k = 0; k < NA; k++) red[k * LMA_RED + lane] = A[k];
 #pragma unroll
-  for (int k = 0; k < LMA_NP; k++) red[(21 + k) * 33 + lane] = b[k];
-  red[27 * 33 + lane] = r2;
+  for (int k = 0; k < NP; k++) red[(NA + k) * LMA_RED + lane] = b[k];
+  red[(NA + NP) * LMA_RED + lane] = r2;
   __syncwarp();
-  if (lane < LMA_NEQ) {
+  if (lane < lma_neq(NP)) {
     float t = 0.f;
-    for (int i = 0; i < 32; i++) t += red[lane * 33 + i];
+    const float4 *row = (const float4 *)(red + lane * LMA_RED);
+    const int n4 = min(ns + 3, 32) >> 2;
+    for (int i = 0; i < n4; i++) {
+      const float4 q = row[i];
+      t += q.x; t += q.y; t += q.z; t += q.w;
+    }
     // the two regularisation samples: WM towards half_width, WXY towards 0
-    const float e1 = half_width - av[1], e2 = -av[3];
-    if (lane == 6) t += w_wm;                 // A (1, 1)
-    if (lane == 15) t += w_wxy;               // A (3, 3)
-    if (lane == 22) t += w_wm * e1;           // b 1
-    if (lane == 24) t += w_wxy * e2;          // b 3
-    if (lane == 27) t += w_wm * e1 * e1 + w_wxy * e2 * e2;
+    const float e1 = half_width - av[1], e2 = -av[Par::wxy];
+    if (lane == NP) t += w_wm;                    // A (1, 1)
+    if (lane == Par::wxy2) t += w_wxy;            // A (wxy, wxy)
+    if (lane == NA + 1) t += w_wm * e1;           // b 1
+    if (lane == NA + Par::wxy) t += w_wxy * e2;   // b wxy
+    if (lane == NA + NP) t += w_wm * e1 * e1 + w_wxy * e2 * e2;
     out[lane] = t;
   }
   __syncwarp();
@@ -218,7 +234,7 @@ __device__ __forceinline__ void lma_eval(const float *sx, const float *sy, const
 
 }  // namespace
 
-// One Correlation2d.corrLMA fit of a tile from the staged pair surfaces `src` ([P][225]) of the
+// One Correlation2d.corrLMA fit of a tile from the pair surfaces `src` ([P][225]) of the
 // pair kinds in kmask (bit k: kind k), centred at xcenter: res = {disparity, strength, WM, WXY}
 // (getDisparityStrengthWidth); false when there are no samples or the fit did not converge.
 // Samples of the selected pairs (BY_PAIR: bit = pair index, else bit = pair kind; pairs of kind -1
@@ -241,31 +257,50 @@ __device__ __forceinline__ int lma_samples(const LmaDev &ld, const TpLmaConst &c
     np_ortho += (k <= 1);
     np_diag += (k >= 2);
   }
-  // group sums, pairs in index order (combineCompatiblePairs), 8 cells per lane in registers
+  // group sums, pairs in index order (combineCompatiblePairs), 8 cells per lane in registers; the cells' places in
+  // the pair's surface are worked out once per run of pairs of one kind
   float go[8], gdg[8];
+  int at[8], kprev = -1;
 #pragma unroll
-  for (int t = 0; t < 8; t++) go[t] = gdg[t] = 0.f;
+  for (int t = 0; t < 8; t++) {
+    go[t] = gdg[t] = 0.f;
+    at[t] = 0;
+  }
   for (int pi = 0; pi < ld.P; pi++) {
     const int k = ld.kinds[pi];
     if (k < 0 || !((sel_mask >> (BY_PAIR ? pi : k)) & 1)) continue;
+    if (k != kprev) {
+#pragma unroll
+      for (int t = 0; t < 8; t++) {
+        const int i = min(lane + 32 * t, TP_CORR - 1), r = i / 15, q = i - r * 15;
+        at[t] = (k == 1) ? q * 15 + r : ((k == 3) ? (14 - r) * 15 + q : i);
+      }
+      kprev = k;
+    }
     const float *cs = src + pi * TP_CORR;
+    float v[8];
+#pragma unroll
+    for (int t = 0; t < 8; t++) v[t] = cs[at[t]];
+    if (k >= 2) {
+#pragma unroll
+      for (int t = 0; t < 8; t++) gdg[t] += v[t];
+    } else {
+#pragma unroll
+      for (int t = 0; t < 8; t++) go[t] += v[t];
+    }
+  }
+  // the means; the reciprocal of 1, 2, 4, ... is exact, so the product is the quotient
+#pragma unroll
+  for (int gd = 0; gd < 2; gd++) {
+    const int npg = gd ? np_diag : np_ortho;
+    if (npg == 0) continue;  // not read
+    const float inv = 1.0f / npg;
+    const bool exact = (npg & (npg - 1)) == 0;
 #pragma unroll
     for (int t = 0; t < 8; t++) {
       const int i = lane + 32 * t;
-      if (i < 225) {
-        const int r = i / 15, q = i - r * 15;
-        const float v = (k == 1) ? cs[q * 15 + r] : ((k == 3) ? cs[(14 - r) * 15 + q] : cs[i]);
-        if (k >= 2) gdg[t] += v;
-        else go[t] += v;
-      }
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < 8; t++) {
-    const int i = lane + 32 * t;
-    if (i < 225) {
-      gsurf[i] = (np_ortho > 1) ? go[t] / np_ortho : go[t];
-      gsurf[225 + i] = (np_diag > 1) ? gdg[t] / np_diag : gdg[t];
+      const float g = gd ? gdg[t] : go[t];
+      if (i < TP_CORR) gsurf[TP_CORR * gd + i] = exact ? g * inv : g / npg;
     }
   }
   __syncwarp();
@@ -395,10 +430,13 @@ __device__ __forceinline__ int lma_samples(const LmaDev &ld, const TpLmaConst &c
 
 // Correlation2d.corrLMA (1754-1877) on the pairs of the kinds in kmask: samples, then the
 // Levenberg-Marquardt fit; res = {disparity, strength, WM, WXY}
+template <bool WY, bool TWO>
 __device__ __forceinline__ bool lma_fit(const LmaDev &ld, const TpLmaConst &c, int kmask, float xcenter,
                                         const float *src, float *gsurf, float *sx, float *sy, float *sv, float *sw,
                                         unsigned char *sg, float *red, float *acc, float *trial, int lane,
                                         float res[4]) {
+  using Par = LmaPar<WY, TWO>;
+  constexpr int NP = Par::n, NA = Par::na;
   int ngroups, gdiag_bits;
   const int ns = lma_samples<false>(ld, c, (unsigned)kmask, xcenter, c.ortho_vasw_pwr, src, gsurf, sx, sy, sv, sw, sg,
                                     lane, ngroups, gdiag_bits);
@@ -432,10 +470,24 @@ __device__ __forceinline__ bool lma_fit(const LmaDev &ld, const TpLmaConst &c, i
   __syncwarp();
   const float w_wm = c.cost_wy * inv, w_wxy = c.cost_wxy * inv;
   const float gwt[2] = {pure > 0.f ? gw0 / pure : gw0, pure > 0.f ? gw1 / pure : gw1};
-  const bool mask[LMA_NP] = {true, c.adjust_wm != 0, c.adjust_wy != 0, c.adjust_wxy != 0,
-                             c.adjust_ag != 0 && ngroups > 0, c.adjust_ag != 0 && ngroups > 1};
-  float av[LMA_NP] = {xcenter, c.half_width, 0.f, 0.f, vmax, vmax};
-  if (ngroups < 2) av[5] = 0.f;
+  bool mask[NP];
+  float av[NP];
+  mask[0] = true;
+  av[0] = xcenter;
+  mask[1] = c.adjust_wm != 0;
+  av[1] = c.half_width;
+  if (WY) {
+    mask[2] = true;
+    av[2] = 0.f;
+  }
+  mask[Par::wxy] = c.adjust_wxy != 0;
+  av[Par::wxy] = 0.f;
+  mask[Par::ag] = c.adjust_ag != 0 && ngroups > 0;
+  av[Par::ag] = vmax;
+  if (TWO) {
+    mask[NP - 1] = c.adjust_ag != 0 && ngroups > 1;
+    av[NP - 1] = (ngroups < 2) ? 0.f : vmax;
+  }
   // ---- runLma / lmaStep ----
   // acc: normal equations at the accepted parameters; trial: at the proposed ones
   // iteration -1 evaluates the start (into acc); one inlined evaluation serves all
@@ -443,21 +495,21 @@ __device__ __forceinline__ bool lma_fit(const LmaDev &ld, const TpLmaConst &c, i
   float lambda = c.lambda_initial;
   bool success = false;
   for (int iter = -1; iter < c.num_iter; iter++) {
-    float nav[LMA_NP];
+    float nav[NP];
     if (iter < 0) {
 #pragma unroll
-      for (int a = 0; a < LMA_NP; a++) nav[a] = av[a];
+      for (int a = 0; a < NP; a++) nav[a] = av[a];
     } else {
       // (JtJ + lambda diag JtJ) delta = Jt W (y - f), masked parameters held (identity rows).
       // The matrix is symmetric positive (semi)definite: LDL^T without pivoting; a pivot that is
       // not positive marks it singular, as the zero pivot of the reference's LU inverse does.
-      float M[LMA_NP][LMA_NP], rhs[LMA_NP];
+      float M[NP][NP], rhs[NP];
       {
         int k = 0;
 #pragma unroll
-        for (int a = 0; a < LMA_NP; a++)
+        for (int a = 0; a < NP; a++)
 #pragma unroll
-          for (int cc = a; cc < LMA_NP; cc++) {
+          for (int cc = a; cc < NP; cc++) {
             const bool keep = mask[a] && mask[cc];
             const float v = keep ? acc[k] : ((a == cc) ? 1.0f : 0.0f);
             M[a][cc] = v;
@@ -466,14 +518,14 @@ __device__ __forceinline__ bool lma_fit(const LmaDev &ld, const TpLmaConst &c, i
           }
       }
 #pragma unroll
-      for (int a = 0; a < LMA_NP; a++) {
+      for (int a = 0; a < NP; a++) {
         if (mask[a]) M[a][a] += M[a][a] * lambda;
-        rhs[a] = mask[a] ? acc[21 + a] : 0.0f;
+        rhs[a] = mask[a] ? acc[NA + a] : 0.0f;
       }
-      float Lm[LMA_NP][LMA_NP], Dd[LMA_NP], Dinv[LMA_NP];
+      float Lm[NP][NP], Dd[NP], Dinv[NP];
       bool singular = false;
 #pragma unroll
-      for (int r = 0; r < LMA_NP; r++) {
+      for (int r = 0; r < NP; r++) {
 #pragma unroll
         for (int cc = 0; cc < r; cc++) {
           float t = M[r][cc];
@@ -489,38 +541,38 @@ __device__ __forceinline__ bool lma_fit(const LmaDev &ld, const TpLmaConst &c, i
         Dinv[r] = (dd > 0.0f) ? 1.0f / dd : 0.0f;
       }
       if (singular) break;
-      float delta[LMA_NP];
+      float delta[NP];
 #pragma unroll
-      for (int r = 0; r < LMA_NP; r++) {
+      for (int r = 0; r < NP; r++) {
         float t = rhs[r];
 #pragma unroll
         for (int k = 0; k < r; k++) t -= Lm[r][k] * delta[k];
         delta[r] = t;
       }
 #pragma unroll
-      for (int r = LMA_NP - 1; r >= 0; r--) {
+      for (int r = NP - 1; r >= 0; r--) {
         float t = delta[r] * Dinv[r];
 #pragma unroll
-        for (int k = r + 1; k < LMA_NP; k++) t -= Lm[k][r] * delta[k];
+        for (int k = r + 1; k < NP; k++) t -= Lm[k][r] * delta[k];
         delta[r] = t;
       }
 #pragma unroll
-      for (int a = 0; a < LMA_NP; a++) nav[a] = av[a] + (mask[a] ? delta[a] : 0.0f);
+      for (int a = 0; a < NP; a++) nav[a] = av[a] + (mask[a] ? delta[a] : 0.0f);
     }
-    lma_eval(sx, sy, sv, sw, sg, gdiag_bits, ns, nav, w_wm, w_wxy, c.half_width, red, iter < 0 ? acc : trial, lane);
+    lma_eval<WY, TWO>(sx, sy, sv, sw, sg, gdiag_bits, ns, nav, w_wm, w_wxy, c.half_width, red, iter < 0 ? acc : trial, lane);
     if (iter < 0) {
-      last = initial = sqrtf(acc[27]);
+      last = initial = sqrtf(acc[NA + NP]);
       continue;
     }
-    const float rms = sqrtf(trial[27]);
+    const float rms = sqrtf(trial[NA + NP]);
     bool done = false;
     if (rms < last) {
       success = true;
       done = rms >= last * (1.0f - c.rms_diff);
       last = rms;
 #pragma unroll
-      for (int a = 0; a < LMA_NP; a++) av[a] = nav[a];
-      if (lane < LMA_NEQ) acc[lane] = trial[lane];
+      for (int a = 0; a < NP; a++) av[a] = nav[a];
+      if (lane < lma_neq(NP)) acc[lane] = trial[lane];
       __syncwarp();
     } else {
       success = false;
@@ -535,12 +587,12 @@ __device__ __forceinline__ bool lma_fit(const LmaDev &ld, const TpLmaConst &c, i
   if (!success && last < initial) success = true;
   if (!success) return false;
   // ---- getDisparityStrength(Width) ----
-  float sum_amp = gwt[0] * av[4] + (ngroups > 1 ? gwt[1] * av[5] : 0.0f);
+  float sum_amp = gwt[0] * av[Par::ag] + ((TWO && ngroups > 1) ? gwt[1] * av[NP - 1] : 0.0f);
   if (sum_amp > 1.25f * smax) sum_amp = smax;
   res[0] = -av[0];
   res[1] = sum_amp;
   res[2] = av[1];
-  res[3] = av[3];
+  res[3] = av[Par::wxy];
   return true;
 }
 
@@ -679,157 +731,159 @@ __device__ bool quadric_max(const double *m, int ns, double *dm, double xyv[3]) 
   return true;
 }
 
-// LY_POLY: the instantiation with the polynomial mismatch measure (the other never carries it)
-template <bool LY_POLY>
-__global__ void __launch_bounds__(32 * LMA_NW) lma_kernel(const __grid_constant__ LmaDev ld,
-                                                         const __grid_constant__ TpLmaConst c) {
+// The main fit (corrLMA, all pairs), one warp per tile: where it converges, rec = {disparity, strength, WM, WXY},
+// and with mix_corr_poly the record's disparity and strength are the fit's; else rec stays NaN.  A warp's work is
+// a chain of dependent arithmetic, so residency is what counts: 80 registers a thread and 8.9 KB of shared memory
+// a warp keep 24 warps on an SM (127 registers and the pair surfaces staged in 14 KB: 16).
+template <bool WY>
+__global__ void __launch_bounds__(32 * LMA_NW, 24 / LMA_NW) lma_main_kernel(const __grid_constant__ LmaDev ld,
+                                                                          const __grid_constant__ TpLmaConst c) {
   extern __shared__ float sm[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int task = blockIdx.x * LMA_NW + warp;
+  if (task >= ld.num_tasks) return;
+  const int txy = ld.task_txy[task];
+  const size_t tile = (size_t)(txy >> 16) * ld.tilesX + (txy & 0xffff);
+  float *rec = ld.lma + tile * 4;
+  float *dm = ld.disp + tile * TP_NDISP;
+  const float cm = dm[1], strength0 = dm[2];  // the record's CM disparity and strength
+  if (lane < 4) rec[lane] = CUDART_NAN_F;
+  if (isnan(cm) || !(strength0 > c.min_poly_strength)) return;
   float *gsurf = sm + warp * LMA_PER_WARP;                      // [2][225]
   float *sx = gsurf + 450;                                      // samples
   float *sy = sx + LMA_MAX_SAMPLES, *sv = sy + LMA_MAX_SAMPLES, *sw = sv + LMA_MAX_SAMPLES;
   unsigned char *sg = (unsigned char *)(sw + LMA_MAX_SAMPLES);
-  float *red = gsurf + LMA_OFF_RED;                             // [LMA_NEQ][33] transposed partial sums
-  float *acc = red + LMA_NEQ * 33, *trial = acc + 32;
-  float *stage = gsurf + LMA_OFF_STAGE;                         // [P][225] the tile's pair surfaces
-  float *dres = gsurf + LMA_OFF_RES;                            // [4][4] the orientation fits
-  // quadric moments [LMA_POLY_CHUNK][21] over the reduction buffer and the per-lane solver scratch
-  // [LMA_POLY_CHUNK][LMA_POLY_SCRATCH] over the group surfaces (both free once the fits are done)
-  double *dmom = (double *)(gsurf + ((LMA_OFF_RED + 1) & ~1));
-  double *dsolve = (double *)gsurf;
-  for (int task = blockIdx.x * LMA_NW + warp; task < ld.num_tasks; task += gridDim.x * LMA_NW) {
-    const int txy = ld.task_txy[task];
-    const size_t tile = (size_t)(txy >> 16) * ld.tilesX + (txy & 0xffff);
-    float *rec = ld.lma + tile * 4;
-    float *dm = ld.disp + tile * TP_NDISP;
-    const float cm = dm[1], strength0 = dm[2];  // the record's CM disparity and strength
-    if (lane < 4) rec[lane] = CUDART_NAN_F;
-    if (ld.mismatch)  // {NaN, NaN, 0} unless measured below
-      for (int i = lane; i < 3 * ld.P; i += 32) ld.mismatch[tile * 3 * ld.P + i] = (i % 3 == 2) ? 0.f : CUDART_NAN_F;
-    if (isnan(cm) || !(strength0 > c.min_poly_strength)) continue;
-    // The tile's surfaces are contiguous (P x 900 bytes): copied asynchronously, all in flight at
-    // once, in 8-byte pieces when P is even (the tile's offset is then a multiple of 8 bytes).
-    const float *src = ld.corr + tile * ld.P * TP_CORR;
-    if (ld.P <= LMA_STAGE_PAIRS) {
-      if ((ld.P & 1) == 0) {
-        for (int k = lane; k < ld.P * TP_CORR / 2; k += 32) cp_async8(stage + 2 * k, src + 2 * k);
-      } else {
-        for (int k = lane; k < ld.P * TP_CORR; k += 32) cp_async4(stage + k, src + k);
-      }
-      asm volatile("cp.async.commit_group;\n" ::: "memory");
-      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-      __syncwarp();
-      src = stage;
-    }
-    // fit 0: all pairs (corrLMA); fits 1-4 with fo_correct: one pair orientation each
-    // (corr4dirsLMA), centred at the (mixed) disparity.  One inlined copy of the fit serves all.
-    float main_res[4] = {0.f, 0.f, 0.f, 0.f};
-    float disparity = cm, strength = strength0, cm_out = cm, str_out = strength0;
-    unsigned valid = 0;
-    bool main_ok = false;
-    const bool mism = ld.mismatch != nullptr;
-    for (int f = 0; f < 5; f++) {
-      if (f > 0 && !((c.fo_correct && strength > 0.0f) || mism)) break;
-      if (f > 0 && ld.kind_count[f - 1] == 0) continue;
-      float res[4];
-      const bool ok = lma_fit(ld, c, f ? 1 << (f - 1) : 0xf, f ? -disparity : -cm, src, gsurf, sx, sy, sv, sw, sg,
-                              red, acc, trial, lane, res);
-      if (f == 0) {
-        if (!ok) break;
-        main_ok = true;
+  float *red = gsurf + LMA_OFF_RED;                             // [28][LMA_RED] transposed partial sums
+  float *acc = red + lma_neq(LMA_NP) * LMA_RED, *trial = acc + 32;
+  float res[4];
+  if (!lma_fit<WY, true>(ld, c, 0xf, -cm, ld.corr + tile * ld.P * TP_CORR, gsurf, sx, sy, sv, sw, sg, red, acc, trial,
+                       lane, res))
+    return;
+  if (lane == 0) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) main_res[k] = res[k];
-        if (c.mix_corr_poly) {
-          disparity = cm_out = res[0];
-          strength = str_out = res[1];
-        }
-      } else if (ok) {
-        valid |= 1u << (f - 1);
-        if (lane < 4) dres[(f - 1) * 4 + lane] = (lane == 0) ? res[0] : ((lane == 1) ? res[1] : ((lane == 2) ? res[2] : res[3]));
-      }
+    for (int k = 0; k < 4; k++) rec[k] = res[k];
+    if (c.mix_corr_poly) {
+      dm[1] = res[0];
+      dm[2] = res[1];
     }
-    if (!main_ok) continue;
-    __syncwarp();
-    if ((c.fo_correct && strength > 0.0f) || mism) {  // foregroundCorrect (ImageDtt.java:2294-2418)
-      float dd[4][4];
-      bool vb[4];
-#pragma unroll
-      for (int d = 0; d < 4; d++) {
-        vb[d] = (valid >> d) & 1;
-#pragma unroll
-        for (int k = 0; k < 4; k++) dd[d][k] = dres[d * 4 + k];
-      }
-      float spread;
-      const float mod = foreground_correct(c, dd, vb, disparity, spread);
-      // the corrected distance is not used while the mismatch is measured
-      if (!mism && c.fo_correct && mod != disparity && strength > c.fo_min_strength) cm_out = mod;
-      if (mism && spread <= c.mismatch_max_diff) {
-        bool need_cm = true;
-        if (LY_POLY) {
-          // ImageDtt.java:2349-2383: each pair alone (mismatchPairs 1434-1503), the quadric's
-          // maximum; an implausible offset zeroes the pair's strength, and with the backup any
-          // failed or implausible pair sends the tile to the centre-of-mass measure
-          // Pairs go in chunks: the warp samples each pair and reduces its moments, then lane j
-          // solves the chunk's j-th pair (the solves are serial FP64 work, so one per lane).
-          bool has_nan = false;
-          const double xc = -(double)disparity;
-          for (int c0 = 0; c0 < ld.P; c0 += LMA_POLY_CHUNK) {
-            const int c1 = min(c0 + LMA_POLY_CHUNK, ld.P);
-            int my_ns = 0;
-            for (int pi = c0; pi < c1; pi++) {
-              if (ld.kinds[pi] < 0) continue;
-              int ng, gdb;
-              const int ns = lma_samples<true>(ld, c, 1u << pi, -disparity, c.max_corr_radius, src, gsurf, sx, sy, sv,
-                                               sw, sg, lane, ng, gdb);
-              quadric_moments(sx, sy, sv, sw, ns, lane, dmom + (pi - c0) * 21);
-              if (lane == pi - c0) my_ns = ns;
-              __syncwarp();  // the next pair's samples overwrite these; the moments are written
-            }
-            const int pi = c0 + lane;
-            bool bad = false;
-            if (pi < c1 && ld.kinds[pi] >= 0) {
-              const int k = ld.kinds[pi];
-              double q[3], o0 = CUDART_NAN, o1 = CUDART_NAN, o2 = 0.0;
-              if (quadric_max(dmom + lane * 21, my_ns, dsolve + lane * LMA_POLY_SCRATCH, q)) {
-                if (k == 0) { o0 = xc - q[0]; o1 = -q[1]; }
-                else if (k == 1) { o0 = -q[1]; o1 = xc - q[0]; }
-                else if (k == 2) { o0 = xc - q[0] + q[1]; o1 = xc - q[0] - q[1]; }
-                else { o0 = xc - q[0] + q[1]; o1 = -xc + q[0] + q[1]; }
-                o2 = isnan(q[2]) ? 0.0 : q[2];
-              }
-              if (isnan(o0) || isnan(o1)) bad = true;
-              else if (o2 != 0.0 && (fabs(o0) > c.ly_crazy_poly || fabs(o1) > c.ly_crazy_poly)) {
-                o2 = 0.0;
-                bad = true;
-              }
-              float *mo = ld.mismatch + (tile * ld.P + pi) * 3;
-              mo[0] = (float)o0;
-              mo[1] = (float)o1;
-              mo[2] = (float)o2;
-            }
-            has_nan |= __any_sync(0xffffffffu, bad);
-            __syncwarp();  // the scratch lies over the next chunk's group surfaces
-          }
-          need_cm = c.ly_poly_backup && has_nan;
-          __syncwarp();
-        }
-        if (need_cm && lane < ld.P && ld.kinds[lane] >= 0) {
-          float m3[3];
-          mismatch_cm(src + lane * TP_CORR, ld.kinds[lane], -disparity, c.max_corr_radius, m3);
-          float *mo = ld.mismatch + (tile * ld.P + lane) * 3;
-          mo[0] = m3[0];
-          mo[1] = m3[1];
-          mo[2] = m3[2];
-        }
-      }
-    }
+  }
+}
+
+// The four orientation fits (corr4dirsLMA) of a tile whose main fit converged, centred at the (mixed) disparity,
+// one warp each, and what follows from them: foregroundCorrect and the lazy-eye mismatch of the pairs.  A fit of
+// one orientation has one group, so five parameters.  In a launch of its own with a CTA per tile: as the second
+// to fifth fit of the main fit's warp they left the chip half empty in the last wave.  4 x 648x488 (4,941 tiles):
+// 180 us for all five fits in one warp, 164 at 24 warps an SM, 35 + 89 in two launches, 32 + 76 without WYD's row
+// and with the pairs' cells worked out once per kind.
+// LY_POLY: the instantiation with the polynomial mismatch measure (the other never carries it).
+template <bool LY_POLY, bool WY>
+__global__ void __launch_bounds__(32 * LMA_DIRS, LY_POLY ? 1 : 6) lma_dirs_kernel(const __grid_constant__ LmaDev ld,
+                                                                                const __grid_constant__ TpLmaConst c) {
+  extern __shared__ float sm[];
+  __shared__ float dres[LMA_DIRS][4];  // the orientation fits
+  __shared__ int dvalid[LMA_DIRS], pair_ns[LMA_POLY_CHUNK];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int txy = ld.task_txy[blockIdx.x];
+  const size_t tile = (size_t)(txy >> 16) * ld.tilesX + (txy & 0xffff);
+  if (isnan(ld.lma[tile * 4])) return;  // no main fit
+  float *dm = ld.disp + tile * TP_NDISP;
+  const float disparity = dm[1], strength = dm[2];
+  const bool mism = ld.mismatch != nullptr;
+  if (!(strength > 0.0f) && !mism) return;
+  const float *src = ld.corr + tile * ld.P * TP_CORR;
+  float *gsurf = sm + warp * LMA_PER_WARP;                      // [2][225]
+  float *sx = gsurf + 450;                                      // samples
+  float *sy = sx + LMA_MAX_SAMPLES, *sv = sy + LMA_MAX_SAMPLES, *sw = sv + LMA_MAX_SAMPLES;
+  unsigned char *sg = (unsigned char *)(sw + LMA_MAX_SAMPLES);
+  float *red = gsurf + LMA_OFF_RED;                             // [28][LMA_RED] transposed partial sums
+  float *acc = red + lma_neq(LMA_NP) * LMA_RED, *trial = acc + 32;
+  // quadric moments [LMA_POLY_CHUNK][21] over warp 0's reduction buffer and the per-lane solver scratch
+  // [LMA_POLY_CHUNK][LMA_POLY_SCRATCH] over its group surfaces (both free once the fits are done)
+  double *dmom = (double *)(sm + ((LMA_OFF_RED + 1) & ~1));
+  double *dsolve = (double *)sm;
+  {
+    float res[4];
+    const bool ok = ld.kind_count[warp] != 0 && lma_fit<WY, false>(ld, c, 1 << warp, -disparity, src, gsurf, sx, sy, sv,
+                                                                     sw, sg, red, acc, trial, lane, res);
     if (lane == 0) {
-      rec[0] = main_res[0];
-      rec[1] = main_res[1];
-      rec[2] = main_res[2];
-      rec[3] = main_res[3];
-      dm[1] = cm_out;
-      dm[2] = str_out;
+      dvalid[warp] = ok;
+      if (ok)
+#pragma unroll
+        for (int k = 0; k < 4; k++) dres[warp][k] = res[k];
+    }
+  }
+  __syncthreads();
+  if (warp && !(LY_POLY && mism)) return;
+  // foregroundCorrect (ImageDtt.java:2294-2418)
+  float dd[4][4];
+  bool vb[4];
+#pragma unroll
+  for (int d = 0; d < 4; d++) {
+    vb[d] = dvalid[d];
+#pragma unroll
+    for (int k = 0; k < 4; k++) dd[d][k] = vb[d] ? dres[d][k] : 0.f;
+  }
+  float spread;
+  const float mod = foreground_correct(c, dd, vb, disparity, spread);
+  // the corrected distance is not used while the mismatch is measured
+  if (!mism && lane == 0 && mod != disparity && strength > c.fo_min_strength) dm[1] = mod;
+  if (mism && spread <= c.mismatch_max_diff) {
+    bool need_cm = true;
+    if (LY_POLY) {
+      // ImageDtt.java:2349-2383: each pair alone (mismatchPairs 1434-1503), the quadric's
+      // maximum; an implausible offset zeroes the pair's strength, and with the backup any
+      // failed or implausible pair sends the tile to the centre-of-mass measure
+      // Pairs go in chunks: each warp samples pairs and reduces their moments, then lane j of
+      // warp 0 solves the chunk's j-th pair (the solves are serial FP64 work, so one per lane).
+      bool has_nan = false;
+      const double xc = -(double)disparity;
+      for (int c0 = 0; c0 < ld.P; c0 += LMA_POLY_CHUNK) {
+        const int c1 = min(c0 + LMA_POLY_CHUNK, ld.P);
+        for (int pi = c0 + warp; pi < c1; pi += LMA_DIRS) {
+          if (ld.kinds[pi] < 0) continue;
+          int ng, gdb;
+          const int ns = lma_samples<true>(ld, c, 1u << pi, -disparity, c.max_corr_radius, src, gsurf, sx, sy, sv,
+                                           sw, sg, lane, ng, gdb);
+          quadric_moments(sx, sy, sv, sw, ns, lane, dmom + (pi - c0) * 21);
+          if (lane == 0) pair_ns[pi - c0] = ns;
+          __syncwarp();  // the next pair's samples overwrite these; the moments are written
+        }
+        __syncthreads();  // every warp's moments
+        const int pi = c0 + lane;
+        bool bad = false;
+        if (warp == 0 && pi < c1 && ld.kinds[pi] >= 0) {
+          const int k = ld.kinds[pi];
+          double q[3], o0 = CUDART_NAN, o1 = CUDART_NAN, o2 = 0.0;
+          if (quadric_max(dmom + lane * 21, pair_ns[lane], dsolve + lane * LMA_POLY_SCRATCH, q)) {
+            if (k == 0) { o0 = xc - q[0]; o1 = -q[1]; }
+            else if (k == 1) { o0 = -q[1]; o1 = xc - q[0]; }
+            else if (k == 2) { o0 = xc - q[0] + q[1]; o1 = xc - q[0] - q[1]; }
+            else { o0 = xc - q[0] + q[1]; o1 = -xc + q[0] + q[1]; }
+            o2 = isnan(q[2]) ? 0.0 : q[2];
+          }
+          if (isnan(o0) || isnan(o1)) bad = true;
+          else if (o2 != 0.0 && (fabs(o0) > c.ly_crazy_poly || fabs(o1) > c.ly_crazy_poly)) {
+            o2 = 0.0;
+            bad = true;
+          }
+          float *mo = ld.mismatch + (tile * ld.P + pi) * 3;
+          mo[0] = (float)o0;
+          mo[1] = (float)o1;
+          mo[2] = (float)o2;
+        }
+        has_nan |= __any_sync(0xffffffffu, bad);
+        __syncthreads();  // the scratch lies over the next chunk's moments and group surfaces
+      }
+      need_cm = c.ly_poly_backup && has_nan;
+      __syncwarp();
+    }
+    if (need_cm && warp == 0 && lane < ld.P && ld.kinds[lane] >= 0) {
+      float m3[3];
+      mismatch_cm(src + lane * TP_CORR, ld.kinds[lane], -disparity, c.max_corr_radius, m3);
+      float *mo = ld.mismatch + (tile * ld.P + lane) * 3;
+      mo[0] = m3[0];
+      mo[1] = m3[1];
+      mo[2] = m3[2];
     }
   }
 }
@@ -1001,18 +1055,14 @@ cudaError_t launch_lma(const SceneDev &sc, const CorrConst &cc, const TpLmaConst
     ld.kinds[i] = (k >= 0 && k <= 3 && i < 32 && ((c.pair_mask >> i) & 1)) ? k : -1;  // the mask holds 32 pairs
     if (ld.kinds[i] >= 0) ld.kind_count[ld.kinds[i]]++;
   }
-  const int bytes = lma_smem_bytes();
-  const auto kern = (mismatch_out && c.ly_poly) ? lma_kernel<true> : lma_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e != cudaSuccess) return e;
-  int dev = 0, sms = 152, per_sm = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * LMA_NW, bytes);
-  if (per_sm < 1) return cudaErrorInvalidConfiguration;
-  const int units = (sc.num_tasks + LMA_NW - 1) / LMA_NW;
-  const int grid = units < sms * per_sm ? units : sms * per_sm;
-  kern<<<grid, 32 * LMA_NW, bytes, st>>>(ld, c);
+  const auto main_kern = c.adjust_wy ? lma_main_kernel<true> : lma_main_kernel<false>;
+  main_kern<<<(sc.num_tasks + LMA_NW - 1) / LMA_NW, 32 * LMA_NW, lma_smem_bytes(), st>>>(ld, c);
+  if (c.fo_correct || mismatch_out) {
+    const bool poly = mismatch_out && c.ly_poly;
+    const auto kern = poly ? (c.adjust_wy ? lma_dirs_kernel<true, true> : lma_dirs_kernel<true, false>)
+                           : (c.adjust_wy ? lma_dirs_kernel<false, true> : lma_dirs_kernel<false, false>);
+    kern<<<sc.num_tasks, 32 * LMA_DIRS, LMA_DIRS * LMA_PER_WARP * 4, st>>>(ld, c);
+  }
   return cudaGetLastError();
 }
 

@@ -181,3 +181,38 @@ def test_lma_rejects_general_pairs(oracle):
         tp.process()
         with pytest.raises(_lib.TpError, match="quad kinds"):
             tp.lmaRefine()
+
+
+@pytest.mark.parametrize("params", [
+    dict(),
+    dict(adjust_wy=1, adjust_wm=0),         # six / five parameters with WYD in the place of WM
+    dict(pair_mask=0x03),                   # horizontal pairs only: one group, one orientation
+    dict(pair_mask=0x3e, cost_wxy=0.01),    # five pairs: group means over 3 (a division) and 2
+    dict(adjust_ag=0, adjust_wxy=0, num_iter=1),
+], ids=["default", "wyd", "one_kind", "five_pairs", "held"])
+def test_lma_parameter_sets_match_oracle(oracle, params):
+    """The fits' forms (with and without WYD, one and two groups, held parameters) on an odd number of tiles, main
+    fit and record.  Bounds as above: 0.005 px and 1e-3 relative on >= 97% of the refined tiles."""
+    sc = synth.make_scene("quad_mono", seed=47, width=104, height=72)
+    T = 13 * 9
+    with make_gpu(sc) as tp:
+        tp.setCorrelation()
+        tp.setFullFrameImages(np.full(T, 4.0, np.float32))
+        tp.process()
+        corr, d0 = tp.getCorr(), tp.getDisparity()
+        lma = tp.lmaRefine(**params)
+        d1 = tp.getDisparity()
+    op = oracle.default_lma_params(**params)
+    n = ok = 0
+    for t in range(T):
+        ran, rec, lm = oracle.lma_tile(corr[t].astype(np.float64), KINDS, float(d0[t, oracle.DISP_CM]),
+                                       float(d0[t, oracle.DISP_STRENGTH]), params=op)
+        fit = bool(np.isfinite(lma[t, 0]))
+        if not ran and not fit:
+            assert np.array_equal(d1[t], d0[t], equal_nan=True)
+            continue
+        n += 1
+        ok += (ran and fit and abs(lma[t, 0] - lm[0]) <= 0.005 and abs(d1[t, oracle.DISP_CM] - rec[0]) <= 0.005 and
+               abs(d1[t, oracle.DISP_STRENGTH] - rec[1]) <= 1e-3 * abs(rec[1]) + 1e-6)
+    assert n > 20
+    assert ok >= 0.97 * n, "main fit and record agree on %d of %d tiles" % (ok, n)
