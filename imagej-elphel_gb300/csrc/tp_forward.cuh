@@ -36,6 +36,7 @@ __device__ __forceinline__ void subtile_clt(const PIX &w, float rx, float ry, in
       const float hk = b1 ? fh.sc1 * hw1[j] : fh.sc0 * hw0[j];
       y[j] = (vk * hk) * w.at(srow, scol);
     }
+    __syncwarp();  // every window is read: the transpose buffers may lie over them
     float z[8];
     dct4_fast(y, z);
     group_transpose(z, tbuf, r);
@@ -509,18 +510,20 @@ __device__ __forceinline__ void fwd_extract(const SceneDev &sc, const CorrConst 
 // corner.  The fold then reads shared memory; read from global memory, each of its loads touches 32
 // image rows, one L1 access each.  Image rows start on 16-byte boundaries because the pitch is a
 // multiple of 8 pixels.  Windows that cross the image border are copied pair by pair with the edge mirroring.
-// Rows of u16 windows are 24 pixels (three chunks); rows of float windows 20 (five chunks), the
-// sensors' windows 4 floats apart in bank so that the fold's reads spread over the banks.
+// Rows of u16 windows are 24 pixels (three chunks); rows of float windows 20 (five chunks).  The sensors' windows
+// lie 8 banks apart, so that a dense fold's reads (eight rows of four sensors) meet in a bank 3.4 times on average
+// over the corners' positions (u16 without the 8 floats 4.2; even and odd rows apart 2.2, but that costs more
+// instructions than it saves accesses: 693 -> 705 us at 4 x 2592x1936).
 // ---------------------------------------------------------------------------
 template <bool U16>
 struct Stage {
   using T = float;
-  static constexpr int CH = 4, NCH = 5, ROW = 20, WIN = 324;  // pixels per chunk, chunks per row, row, window (floats)
+  static constexpr int CH = 4, NCH = 5, ROW = 20, WIN = 328;  // pixels per chunk, chunks per row, row, window (floats)
 };
 template <>
 struct Stage<true> {
   using T = uint16_t;
-  static constexpr int CH = 8, NCH = 3, ROW = 24, WIN = 192;
+  static constexpr int CH = 8, NCH = 3, ROW = 24, WIN = 200;
 };
 
 __device__ __forceinline__ void cp_async16(void *dst_smem, const void *src) {

@@ -104,15 +104,36 @@ __device__ __forceinline__ void bulk_done() { asm volatile("cp.async.bulk.wait_g
 // of one tile by one warp.  Each sensor's coefficients are read once for the six pairs (the scalar
 // phase reads them three times) and squared once; then the six spectra are kept as three
 // interleaved couples [4][8][9] of float2 over the space of the CLT, which is no longer needed.
-// ws: the warp's region of QP_FLOATS or more floats, the CLT [C][4][256] first.
+// ws: the warp's region of QP_FLOATS or more floats, the CLT [C][4][QP_CLT] first; it is stored to HBM here too.
 // surfaces (15x15, six in a row) go to `surf` and from there to HBM in one asynchronous copy.
 // ---------------------------------------------------------------------------
+// The CLT of a (colour, sensor) here: four quadrants of two half quadrants (rows 0-3, rows 4-7), each 32 values
+// and then 4 unused ones, so that eight lanes that store a row each, 16 bytes at a time, reach different banks.
+constexpr int QP_HALF = 36, QP_QUAD = 68, QP_CLT = 4 * QP_QUAD;  // floats to the second half, the next quadrant, sensor
 constexpr int QP_BUF = 576;                       // floats of one couple's spectra
 constexpr int QP_SURF = 3 * QP_BUF;               // first surface (+ 2 floats for odd tiles)
 constexpr int QP_FLOATS = QP_SURF + 2 + 6 * 225 + 4;  // rounded to 16 bytes: 3084
 
+// store_clt for a sensor of colour c, from the lanes' values of CLT indices l and l + 32: 128 contiguous bytes a store
+// (a row a lane, 16 bytes at a time, each store touches half of 32 sectors)
 template <int C>
-__device__ __forceinline__ void quad_spectra(const CorrConst &cfg, const float *lpf, float *ws, int lane) {
+__device__ __forceinline__ void store_clt_lanes(const SceneDev &sc, int c, size_t tile, int cam, const float2 d[4],
+                                                int lane) {
+  float *g = sc.clt + ((tile * 4 + cam) * C + c) * TP_CLT + lane;
+  float2 l = make_float2(1.f, 1.f);  // exact
+  if (sc.lpf_rbg && ((sc.clt_lpf_mask >> c) & 1))
+    l = make_float2(__ldg(sc.lpf_rbg + c * 64 + lane), __ldg(sc.lpf_rbg + c * 64 + 32 + lane));
+#pragma unroll
+  for (int m = 0; m < 4; m++) {
+    const float2 v = mul2(d[m], l);
+    g[m * 64] = v.x;
+    g[m * 64 + 32] = v.y;
+  }
+}
+
+template <int C>
+__device__ __forceinline__ void quad_spectra(const SceneDev &sc, const CorrConst &cfg, const float *lpf, size_t tile,
+                                             float *ws, int lane) {
   // The loops over colours and couples stay loops: unrolled, a tile's straight-line code misses the
   // instruction cache (the 16 warps of an SM are all at different places of it).
   float2 acc[6][4];
@@ -125,13 +146,15 @@ __device__ __forceinline__ void quad_spectra(const CorrConst &cfg, const float *
     float2 d[4][4], s[4];
 #pragma unroll
     for (int cam = 0; cam < 4; cam++) {
-      const float *p = ws + (c * 4 + cam) * TP_CLT + lane;
+      const float *p = ws + (c * 4 + cam) * QP_CLT + lane;
 #pragma unroll
-      for (int m = 0; m < 4; m++) d[cam][m] = make_float2(p[m * 64], p[m * 64 + 32]);
+      for (int m = 0; m < 4; m++) d[cam][m] = make_float2(p[m * QP_QUAD], p[m * QP_QUAD + QP_HALF]);
       s[cam] = mul2(d[cam][0], d[cam][0]);
 #pragma unroll
       for (int m = 1; m < 4; m++) s[cam] = fma2(d[cam][m], d[cam][m], s[cam]);
     }
+#pragma unroll
+    for (int cam = 0; cam < 4; cam++) store_clt_lanes<C>(sc, c, tile, cam, d[cam], lane);
     constexpr int c1[6] = {0, 2, 0, 1, 0, 2}, c2[6] = {1, 3, 2, 3, 3, 1};
     float2 a2[6];
     float v[6], fzs[6];
@@ -222,6 +245,66 @@ __device__ __forceinline__ void couple_surfaces(float2 *b, float *s0, float *s1,
   }
 }
 
+// One couple of a standard quad's pairs over C colours: spectra of pairs 2k and 2k + 1 into b ([4][72] float2).
+// clt: [C][4][QP_CLT]; the couple's sensors f0, g0 and f1, g1.  The CLT of colour `keep` is stored to HBM.  l: the
+// LPF at l and l + 32, over four (the unfold's factor).
+template <int C>
+__device__ __forceinline__ void couple_of_quad(const SceneDev &sc, const CorrConst &cfg, float2 l, const float *clt,
+                                               size_t tile, int keep, int f0, int g0, int f1, int g1, float2 *b, int lane) {
+  float2 acc[2][4];
+#pragma unroll
+  for (int h = 0; h < 2; h++)
+#pragma unroll
+    for (int m = 0; m < 4; m++) acc[h][m] = make_float2(0.f, 0.f);
+#pragma unroll 1
+  for (int c = 0; c < C; c++) {
+    const float *cc = clt + c * 4 * QP_CLT + lane;
+    float2 t[2][4], a2[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int sf = h ? f1 : f0, sg = h ? g1 : g0;
+      const float *pf = cc + sf * QP_CLT, *pg = cc + sg * QP_CLT;
+      float2 x[4], y[4], n[4];
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        x[m] = make_float2(pf[m * QP_QUAD], pf[m * QP_QUAD + QP_HALF]);
+        y[m] = make_float2(pg[m * QP_QUAD], pg[m * QP_QUAD + QP_HALF]);
+      }
+      if (c == keep) {
+        store_clt_lanes<C>(sc, c, tile, sf, x, lane);
+        store_clt_lanes<C>(sc, c, tile, sg, y, lane);
+      }
+      float2 sx = mul2(x[0], x[0]), sy = mul2(y[0], y[0]);
+#pragma unroll
+      for (int m = 1; m < 4; m++) {
+        sx = fma2(x[m], x[m], sx);
+        sy = fma2(y[m], y[m], sy);
+        n[m] = neg2(x[m]);
+      }
+      const float2 pr = mul2(sx, sy);
+      a2[h] = make_float2(amp_of(pr.x), amp_of(pr.y));
+      clt_products(x, n, y, t[h]);
+    }
+    const float2 fzs = warp_sum2(make_float2(a2[0].x + a2[0].y, a2[1].x + a2[1].y), lane, 1.0f / 64, cfg.fat_zero);
+    const float wgt = (C == 1) ? 1.0f : cfg.col_weights[c];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const float2 den = fma2(dup2(h ? fzs.y : fzs.x), dup2(cfg.fat_zero), a2[h]);
+      const float2 sw = make_float2(__fdividef(wgt, den.x), __fdividef(wgt, den.y));
+#pragma unroll
+      for (int m = 0; m < 4; m++) acc[h][m] = fma2(t[h][m], sw, acc[h][m]);
+    }
+  }
+  b += (lane >> 3) * 9 + (lane & 7);
+#pragma unroll
+  for (int m = 0; m < 4; m++) {
+    const float2 x = mul2(acc[0][m], l), y = mul2(acc[1][m], l);
+    b[m * 72] = make_float2(x.x, y.x);
+    b[m * 72 + 36] = make_float2(x.y, y.y);
+  }
+  __syncwarp();
+}
+
 // sample of a strip entry: sample_code of the two sides, averaged below the first row
 __device__ __forceinline__ float strip_of(const float *c, short2 code, int e) {
   float d = sample_code(c, code.x);
@@ -242,7 +325,7 @@ __device__ __forceinline__ short2 quad_code(const short *strip_code, int kind, i
 template <int C>
 __device__ __forceinline__ const float *quad_surfaces(const SceneDev &sc, const CorrConst &cfg, const float *lpf,
                                                       size_t tile, float *ws, int lane) {
-  quad_spectra<C>(cfg, lpf, ws, lane);
+  quad_spectra<C>(sc, cfg, lpf, tile, ws, lane);
   if (C == 1) {  // the last tile's surfaces are out (with colours the caller has waited already)
     if (lane == 0) bulk_read_done();
     __syncwarp();

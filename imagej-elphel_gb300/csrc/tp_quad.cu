@@ -4,16 +4,16 @@
 // A warp carries a tile through all stages, as in the general warp-per-tile schedule, with three
 // differences: the image windows are staged in shared memory one item ahead (tp_forward.cuh), the
 // six pairs are taken together two values per instruction (tp_pairs.cuh), and the extraction's serial
-// half runs as a pass of its own (extract_kernel).
+// half runs as a pass of its own (extract_kernel).  u16 Bayer tiles with short strips are shared by three warps
+// (quad3_kernel).
 //
-// Measured (kernel and extraction together, before -> now): 4x2592x1936 u16 Bayer with kernel tables,
-// 78,408 tiles: 0.922 -> 0.813 ms; 4x1304x984 float Bayer, 7,018 tiles: 129 -> 82 us; 16 batched
-// 4x512x384 float mono scenes, 49,152 tiles: 452 -> 334 us.  What bounds it now: latency at 16 warps
-// an SM (128 registers a thread): the issue slots are about half used, the shared-memory pipe
-// 60 % (Bayer) to 68 % (mono).
+// Measured (kernel and extraction together, general schedule -> now): 4x2592x1936 u16 Bayer with kernel
+// tables, 78,408 tiles: 0.922 -> 0.756 ms; 4x1304x984 float Bayer, 7,018 tiles: 129 -> 80 us; 16 batched
+// 4x512x384 float mono scenes, 49,152 tiles: 452 -> 316 us.  What bounds it now: latency at 16 warps
+// an SM (128 registers a thread): the issue slots and the shared-memory pipe are a little over half used.
 //
-// Shared memory of a warp (floats): CLT [C][4 sensors][256] first; the windows of colour item c at
-// 1024 c (where that item's CLT goes once they are read); the pairs' spectra over the CLT
+// Shared memory of a warp (floats): CLT [C][4 sensors][QP_CLT] first; the windows of colour item c at
+// 4 QP_CLT c (where that item's CLT goes once they are read); the pairs' spectra over the CLT
 // (QP_SURF floats), then the surfaces; transpose buffers behind the CLT.
 #include "tp_forward.cuh"
 #include "tp_pairs.cuh"
@@ -21,8 +21,8 @@
 
 namespace {
 
-__host__ __device__ constexpr int quad_warp_floats(int C) { return C == 3 ? 3 * 1024 + SCR : QP_FLOATS; }
-__host__ __device__ constexpr int quad_tbuf(int C) { return C == 3 ? 3 * 1024 : 1300; }
+__host__ __device__ constexpr int quad_warp_floats(int C) { return C == 3 ? 12 * QP_CLT + SCR : QP_FLOATS; }
+__host__ __device__ constexpr int quad_tbuf(int C) { return C == 3 ? 12 * QP_CLT : 4 * Stage<false>::WIN; }
 
 __device__ __forceinline__ SubtilePlan quad_plan(const SceneDev &sc, int C, int task, int s, int c) {
   return sc.plan[((size_t)task * 4 + s) * C + c];
@@ -31,13 +31,13 @@ __device__ __forceinline__ SubtilePlan quad_plan(const SceneDev &sc, int C, int 
 // lane q * 8 + r copies its share of sensor q's window of colour item c
 template <bool U16>
 __device__ __forceinline__ void quad_stage(const SceneDev &sc, const SubtilePlan &p, int c, float *ws, int q, int r) {
-  stage_window<U16>(sc, sc.images[q], p.tlx, p.tly, ws + c * 1024 + q * Stage<U16>::WIN, r);
+  stage_window<U16>(sc, sc.images[q], p.tlx, p.tly, ws + c * 4 * QP_CLT + q * Stage<U16>::WIN, r);
   cp_async_commit();
 }
 
 // phase A of a tile: p is the plan of (sensor q, colour 0), whose windows are staged
 template <int C, bool U16>
-__device__ __forceinline__ void quad_clt(const SceneDev &sc, int task, size_t tile, SubtilePlan p, float *ws, int lane) {
+__device__ __forceinline__ void quad_clt(const SceneDev &sc, int task, SubtilePlan p, float *ws, int lane) {
   const int q = lane >> 3, r = lane & 7;
   const int rr = sc.bayer_red_row, rc = sc.bayer_red_col;
   float *tbuf = ws + quad_tbuf(C) + q * 72;
@@ -45,7 +45,7 @@ __device__ __forceinline__ void quad_clt(const SceneDev &sc, int task, size_t ti
   for (int c = 0; c < C; c++) {
     const SubtilePlan pn = (c + 1 < C) ? quad_plan(sc, C, task, q, c + 1) : p;
     SWin<U16> w;
-    w.base = (const typename Stage<U16>::T *)(ws + c * 1024 + q * Stage<U16>::WIN);
+    w.base = (const typename Stage<U16>::T *)(ws + c * 4 * QP_CLT + q * Stage<U16>::WIN);
     w.sx = p.tlx & (Stage<U16>::CH - 1);
     w.scale = sc.color_scale[c];
     cp_async_wait_all();  // this item's windows, copied by every lane
@@ -64,13 +64,12 @@ __device__ __forceinline__ void quad_clt(const SceneDev &sc, int task, size_t ti
     if (c + 1 < C) quad_stage<U16>(sc, pn, c + 1, ws, q, r);
     const float *kp = (p.kidx >= 0) ? sc.kernels[q] + (size_t)p.kidx * TP_CLT : nullptr;
     conv_shift(o, kp, p.rx, p.ry, r);
-    float *sdst = ws + (c * 4 + q) * TP_CLT + r * 8;
+    float *sdst = ws + (c * 4 + q) * QP_CLT + r * 8 + (r & 4) * ((QP_HALF - 32) / 4);
 #pragma unroll
     for (int m = 0; m < 4; m++) {
-      *(float4 *)(sdst + m * 64) = make_float4(o[m][0], o[m][1], o[m][2], o[m][3]);
-      *(float4 *)(sdst + m * 64 + 4) = make_float4(o[m][4], o[m][5], o[m][6], o[m][7]);
+      *(float4 *)(sdst + m * QP_QUAD) = make_float4(o[m][0], o[m][1], o[m][2], o[m][3]);
+      *(float4 *)(sdst + m * QP_QUAD + 4) = make_float4(o[m][4], o[m][5], o[m][6], o[m][7]);
     }
-    store_clt(sc, c, r, sc.clt + ((tile * 4 + q) * C + c) * TP_CLT + r * 8, o);
     p = pn;
   }
   __syncwarp();
@@ -117,7 +116,7 @@ __global__ void __launch_bounds__(128, 4) quad_kernel(const __grid_constant__ Sc
     quad_stage<U16>(sc, p, 0, ws, q, r);
   }
   for (; task < sc.num_tasks; task += stride) {
-    quad_clt<C, U16>(sc, task, tile, p, ws, lane);
+    quad_clt<C, U16>(sc, task, p, ws, lane);
     const size_t cur = tile;
     const int next = task + stride;
     if (next < sc.num_tasks) {
@@ -135,6 +134,193 @@ __global__ void __launch_bounds__(128, 4) quad_kernel(const __grid_constant__ Sc
     }
   }
   cp_async_wait_all();
+  if (lane == 0) bulk_done();
+}
+
+// conv_shift (tp_forward.cuh) on two neighbouring values v, v + 1 at a time, the same bits.  buf: 16 floats per
+// eight lanes, where the row's cosines and sines are exchanged.
+__device__ __forceinline__ void conv_shift_pairs(float o[4][8], const float *kp, float rx, float ry, int r, float *buf) {
+  float ch, shh, cvr, svr;
+  __sincosf(CUDART_PI_F * 0.0625f * (2 * r + 1) * rx, &shh, &ch);
+  __sincosf(CUDART_PI_F * 0.0625f * (2 * r + 1) * ry, &svr, &cvr);
+  buf[r] = cvr;
+  buf[8 + r] = svr;
+  __syncwarp();
+  const float2 ch2 = dup2(ch), sh2 = dup2(shh), ns2 = dup2(-shh);
+#pragma unroll
+  for (int w = 0; w < 2; w++) {
+    float4 k[4];
+    if (kp) {
+#pragma unroll
+      for (int m = 0; m < 4; m++) k[m] = __ldg((const float4 *)(kp + m * 64 + r * 8 + 4 * w));
+    }
+    const float4 cq = *(const float4 *)(buf + 4 * w), sq = *(const float4 *)(buf + 8 + 4 * w);
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const int v = 4 * w + 2 * u;
+      float2 d[4];
+#pragma unroll
+      for (int m = 0; m < 4; m++) d[m] = make_float2(o[m][v], o[m][v + 1]);
+      if (kp) {
+        float2 kk[4], n[4];
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+          kk[m] = u ? make_float2(k[m].z, k[m].w) : make_float2(k[m].x, k[m].y);
+          n[m] = neg2(kk[m]);
+        }
+        const float2 e0 = fma2(d[3], kk[3], fma2(d[2], n[2], fma2(d[0], kk[0], mul2(d[1], n[1]))));
+        const float2 e1 = fma2(d[2], n[3], fma2(d[3], n[2], fma2(d[1], kk[0], mul2(d[0], kk[1]))));
+        const float2 e2 = fma2(d[1], n[3], fma2(d[0], kk[2], fma2(d[2], kk[0], mul2(d[3], n[1]))));
+        const float2 e3 = fma2(d[0], kk[3], fma2(d[1], kk[2], fma2(d[3], kk[0], mul2(d[2], kk[1]))));
+        d[0] = e0; d[1] = e1; d[2] = e2; d[3] = e3;
+      }
+      const float2 cv = u ? make_float2(cq.z, cq.w) : make_float2(cq.x, cq.y);
+      const float2 sv = u ? make_float2(sq.z, sq.w) : make_float2(sq.x, sq.y);
+      const float2 nv = neg2(sv);
+      const float2 t0 = fma2(d[0], ch2, mul2(d[1], ns2)), t1 = fma2(d[1], ch2, mul2(d[0], sh2));
+      const float2 t2 = fma2(d[2], ch2, mul2(d[3], ns2)), t3 = fma2(d[3], ch2, mul2(d[2], sh2));
+      const float2 f[4] = {fma2(t0, cv, mul2(t2, nv)), fma2(t1, cv, mul2(t3, nv)), fma2(t0, sv, mul2(t2, cv)),
+                           fma2(t1, sv, mul2(t3, cv))};
+#pragma unroll
+      for (int m = 0; m < 4; m++) {
+        o[m][v] = f[m].x;
+        o[m][v + 1] = f[m].y;
+      }
+    }
+  }
+  __syncwarp();
+}
+
+// u16 Bayer quads with strips of up to 32 entries: three warps per tile.  Phase A: warp k folds colour item k of the
+// four sensors; phase B: warp k carries pairs 2k and 2k + 1 over the three colours to their surfaces and strip
+// values.  A warp needs a third of the registers' and shared memory's contents that it does with a tile to
+// itself, so 24 warps share an SM at 80 registers (warp per tile: 16 at 128).  Two barriers per tile: A, every warp
+// has read the last tile's CLT and written its strip values; B, the CLT is complete.  A warp's own scratch (floats):
+// the staged windows, a tile ahead, then a couple's spectra; behind them its two surfaces, where the folds'
+// transposes go too.
+// 4 x 2592x1936 with kernel tables, 78,408 tiles: warp per tile 729 us, this 728, with conv_shift_pairs
+// 693 (packed, the warp per tile spills: 746); 4 x 648x488, 4,941 tiles: 52 -> 46.  The price is that each warp
+// reads the whole CLT (288 shared-memory accesses a tile instead of 96), so that pipe is at 65 % and the issue
+// slots at 65 %; float windows are too large for eight CTAs an SM (7,018 tiles: 73 us warp per tile, 75 here), so
+// they stay with a warp per tile.
+constexpr int Q3_SURF = 4 * Stage<true>::WIN;       // first surface (+ 0 or 2 floats)
+constexpr int Q3_WS = Q3_SURF + 456;                // scratch of a warp
+constexpr int Q3_FLOATS = 12 * QP_CLT + 3 * Q3_WS;  // 28,896 bytes with the 1 KB a CTA costs: eight in 228 KB
+static_assert(Q3_SURF >= QP_BUF && 8 * (4 * Q3_FLOATS + 1024) <= 228 * 1024, "spectra over the windows, eight CTAs");
+// strip value e of pair p: [6][32] in the 4 unused floats of each of the 48 quadrants
+__device__ __forceinline__ int q3_strip(int p, int e) { return (p * 8 + (e >> 2)) * QP_QUAD + 32 + (e & 3); }
+
+__global__ void __launch_bounds__(96, 8) quad3_kernel(const __grid_constant__ SceneDev sc,
+                                                      const __grid_constant__ CorrConst cfg, int RE) {
+  extern __shared__ float sm[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane >> 3, r = lane & 7;
+  float *ws = sm + 12 * QP_CLT + warp * Q3_WS;
+  const float2 lpf = make_float2(0.25f * cfg.lpf[lane], 0.25f * cfg.lpf[lane + 32]);
+  const int rr = sc.bayer_red_row, rc = sc.bayer_red_col;
+  // the couple's sensors: 0-1 and 2-3, 0-2 and 1-3, 0-3 and 2-1
+  const int f1 = warp == 1 ? 1 : 2, g0 = warp + 1, g1 = warp == 2 ? 1 : 3;
+  // the strip products of a tile: the values are 1 for pairs that are not combined
+  auto products = [&](size_t tile) {
+    if (lane < RE) {
+      float v = sm[q3_strip(0, lane)];
+#pragma unroll
+      for (int p = 1; p < 6; p++) v *= sm[q3_strip(p, lane)];
+      sc.combo[tile * RE + lane] = v;
+    }
+  };
+  int task = blockIdx.x;
+  if (task >= sc.num_tasks) return;
+  SubtilePlan p = quad_plan(sc, 3, task, q, warp);
+  size_t tile = tile_of(sc, task), prev = 0;
+  bool have_prev = false;
+  stage_window<true>(sc, sc.images[q], p.tlx, p.tly, ws + q * Stage<true>::WIN, r);
+  cp_async_commit();
+#pragma unroll 1
+  for (;;) {
+    SWin<true> w;
+    w.base = (const Stage<true>::T *)(ws + q * Stage<true>::WIN);
+    w.sx = p.tlx & (Stage<true>::CH - 1);
+    w.scale = sc.color_scale[warp];
+    cp_async_wait_all();
+    __syncwarp();
+    float o[4][8];
+    float *tbuf = ws + Q3_SURF + q * 72;
+    if (warp < 2) {
+      const int pc = ((warp == 0 ? rc : 1 - rc) - p.tlx) & 1, pr = ((warp == 0 ? rr : 1 - rr) - p.tly) & 1;
+      subtile_clt<1>(w, p.rx, p.ry, pc, pr, 0, r, tbuf, o);
+    } else {
+      const int pg = (p.tlx + p.tly + rc + rr + 1) & 1;
+      subtile_clt<2>(w, p.rx, p.ry, 0, 0, pg, r, tbuf, o);
+    }
+    conv_shift_pairs(o, (p.kidx >= 0) ? sc.kernels[q] + (size_t)p.kidx * TP_CLT : nullptr, p.rx, p.ry, r, tbuf);
+    __syncthreads();  // A
+    float *sdst = sm + (warp * 4 + q) * QP_CLT + r * 8 + (r & 4) * ((QP_HALF - 32) / 4);
+#pragma unroll
+    for (int m = 0; m < 4; m++) {
+      *(float4 *)(sdst + m * QP_QUAD) = make_float4(o[m][0], o[m][1], o[m][2], o[m][3]);
+      *(float4 *)(sdst + m * QP_QUAD + 4) = make_float4(o[m][4], o[m][5], o[m][6], o[m][7]);
+    }
+    if (warp == 2 && have_prev) products(prev);
+    prev = tile;
+    have_prev = true;
+    const int next = task + gridDim.x;
+    const bool more = next < sc.num_tasks;
+    if (more) {
+      p = quad_plan(sc, 3, next, q, warp);
+      tile = tile_of(sc, next);
+    }
+    __syncthreads();  // B
+    couple_of_quad<3>(sc, cfg, lpf, sm, prev, warp, 0, g0, f1, g1, (float2 *)ws, lane);
+    // 1800 bytes from a couple to the next: 0 or 8 past a 16-byte boundary, in shared memory too; the two floats
+    // before or after the aligned 1792 bytes go out by plain stores
+    const int odd = (int)((prev + warp) & 1);
+    float *surf = ws + Q3_SURF + 2 * odd;
+    couple_surfaces((float2 *)ws, surf, surf + 225, lane);
+    bulk_fence();
+    __syncwarp();
+    float *g = sc.corr + prev * 1350 + warp * 450;
+    if (lane == 0) bulk_store(g + 2 * odd, surf + 2 * odd, 1792);
+    if (lane < 2) g[odd ? lane : 448 + lane] = surf[odd ? lane : 448 + lane];
+    if (more) {
+      stage_window<true>(sc, sc.images[q], p.tlx, p.tly, ws + q * Stage<true>::WIN, r);
+      cp_async_commit();
+    }
+    if (warp < 2) {
+      // getMaxXSOrtho profiles of the horizontal (warp 0) and the vertical pairs, as quad_strips: lane j of each
+      // half one column or row, rows 4 half .. 4 half + 3
+      const int half = lane >> 4, j = lane & 15, stride = warp ? 1 : 15;
+      if (j < 15) {
+        const float *lo = surf + (warp ? j * 15 : j) + 4 * half * stride, *hi = lo + (14 - 8 * half) * stride;
+        float pr[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          pr[i] = (0.5f * (lo[0] + hi[0]) + cfg.corr_offset) * (0.5f * (lo[225] + hi[225]) + cfg.corr_offset);
+          lo += stride;
+          hi -= stride;
+        }
+        *(float4 *)(sc.osum + (prev * 32 + warp * 16 + j) * 8 + half * 4) = make_float4(pr[0], pr[1], pr[2], pr[3]);
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int pi = 2 * warp + h;
+      float v = 1.f;
+      if (cfg.pairs[pi].in_combo && lane < RE) {
+        const float d = strip_of(surf + 225 * h, quad_code(&sc.corr_cfg->strip_code[0][0][0], pi < 4 ? pi >> 1 : pi - 2, lane), lane);
+        if (sc.strips) sc.strips[(prev * 6 + pi) * RE + lane] = d;  // kept for the adjoint
+        v = d + cfg.corr_offset;
+        if (v < 0.0f) v = 0.0f;
+        if (cfg.twice_diagonal) v *= v;
+      }
+      sm[q3_strip(pi, lane)] = v;
+    }
+    if (!more) break;
+    if (lane == 0) bulk_read_done();  // the surfaces are out of shared memory
+    __syncwarp();
+    task = next;
+  }
+  __syncthreads();
+  if (warp == 2) products(prev);
   if (lane == 0) bulk_done();
 }
 
@@ -183,7 +369,7 @@ __global__ void __launch_bounds__(128, 4)
         quad_stage<U16>(sc, p, 0, ws, q, r);
       }
       const size_t tile = tile_of(sc, task);
-      quad_clt<1, U16>(sc, task, tile, p, ws, lane);
+      quad_clt<1, U16>(sc, task, p, ws, lane);
       staged = next < sc.num_tasks;  // the next unit's windows, where it is of the same scene
       if (staged) p = quad_plan(sc, 1, next, q, 0);
       const float *surf = quad_surfaces<1>(sc, cfg, cfg.lpf, tile, ws, lane);
@@ -292,13 +478,24 @@ static cudaError_t go_quad(K kernel, int nw, const SceneDev &sc, const CorrConst
   return cudaGetLastError();
 }
 
+static cudaError_t go_quad3(const SceneDev &sc, const CorrConst &cc, int RE, cudaStream_t st) {
+  const int bytes = Q3_FLOATS * 4;
+  int res = 0;
+  const cudaError_t e = kernel_residency((const void *)quad3_kernel, 96, bytes, &res);
+  if (e != cudaSuccess) return e;
+  if (res < 1) return cudaErrorInvalidConfiguration;
+  quad3_kernel<<<sc.num_tasks < res ? sc.num_tasks : res, 96, bytes, st>>>(sc, cc, RE);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_quad_forward(const SceneDev &sc, const CorrConst &cc, int nw, cudaStream_t st) {
   const int RE = strip_entries(sc);
   const bool one = RE <= 32, u16 = sc.img_dtype[0] == 1;
   cudaError_t e;
   if (sc.num_colors == 3) {
-    if (u16) e = one ? go_quad(quad_kernel<3, true, 1>, nw, sc, cc, RE, st) : go_quad(quad_kernel<3, true, 8>, nw, sc, cc, RE, st);
-    else e = one ? go_quad(quad_kernel<3, false, 1>, nw, sc, cc, RE, st) : go_quad(quad_kernel<3, false, 8>, nw, sc, cc, RE, st);
+    if (u16 && one) e = go_quad3(sc, cc, RE, st);
+    else if (one) e = go_quad(quad_kernel<3, false, 1>, nw, sc, cc, RE, st);
+    else e = u16 ? go_quad(quad_kernel<3, true, 8>, nw, sc, cc, RE, st) : go_quad(quad_kernel<3, false, 8>, nw, sc, cc, RE, st);
   } else {
     if (u16) e = one ? go_quad(quad_kernel<1, true, 1>, nw, sc, cc, RE, st) : go_quad(quad_kernel<1, true, 8>, nw, sc, cc, RE, st);
     else e = one ? go_quad(quad_kernel<1, false, 1>, nw, sc, cc, RE, st) : go_quad(quad_kernel<1, false, 8>, nw, sc, cc, RE, st);

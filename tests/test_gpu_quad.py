@@ -95,3 +95,30 @@ def test_quad_batch_matches_single_scenes(u16):
     finally:
         for tp in tps:
             tp.close()
+
+
+@pytest.mark.parametrize("w,h,fill,combo,kw,kern", [
+    (16, 16, 1.0, [1, 1, 1, 1, 1, 1], {}, True),                       # four tiles
+    (24, 200, 1.0, [1, 0, 1, 1, 0, 1], {"twice_diagonal": 0}, False),  # odd and even tiles, pairs not combined
+    (136, 72, 0.4, [0, 1, 1, 0, 1, 1], {}, True),                      # sparse
+    (648, 24, 1.0, [1, 1, 1, 1, 1, 1], {"corr_wndy_size": 1}, True),   # strips of 15 entries
+])
+def test_three_warp_bayer_quads_match_general_path(w, h, fill, combo, kw, kern):
+    """u16 Bayer quads with short strips (a warp per colour, then per couple of pairs) against the general path: the
+    same pairs with one camera's image as float.  The order of operations is the same, so the results are the same
+    bits, the strips' products included."""
+    from tileproc import synth
+    sc = _scene("quad_bayer", True, w, h, 67)
+    T = (w // 8) * (h // 8)
+    rng = np.random.default_rng(11)
+    op = (rng.uniform(size=T) < fill).astype(np.int32)
+    op[0] = op[-1] = 1
+    target = rng.uniform(0, 8, T).astype(np.float32)
+    kernels = synth.random_clt_kernels(rng, 4, h // 16 + 2, w // 16 + 2, 3) if kern else None
+    pairs = [p[:3] + (c,) + p[4:] for p, c in zip(PAIRS, combo)]
+    got = _run(sc, kernels, pairs, op, target, kw)
+    want = _run(sc, kernels, pairs, op, target, kw, mixed=True)
+    on = op != 0
+    assert np.array_equal(got[0][on], want[0][on])
+    assert np.array_equal(got[1][on], want[1][on], equal_nan=True)
+    assert np.array_equal(got[2], want[2], equal_nan=True)
