@@ -24,20 +24,21 @@
 #include <cmath>
 #include <cstdint>
 
-__constant__ float c_dct4[64];   // orthonormal DCT-IV, [k*8+n]
+__constant__ float2 c_dct4p[32];  // orthonormal DCT-IV, outputs k and k + 1: [k/2][n]
 __constant__ float c_dct2e[64];  // DttRad2 CIIe, [j*8+k]
 __constant__ float c_hwin[8];    // sine half-window (DttRad2.set_window(1))
 
 cudaError_t upload_kernel_constants() {
-  float d4[64], d2[64], hw[8];
+  float2 d4[32];
+  float d2[64], hw[8];
   const double pi = 3.14159265358979323846;
   for (int k = 0; k < 8; k++)
     for (int n = 0; n < 8; n++) {
-      d4[k * 8 + n] = (float)(std::sqrt(2.0 / 8) * std::cos(pi * (2 * n + 1) * (2 * k + 1) / 32.0));
+      (k & 1 ? d4[k / 2 * 8 + n].y : d4[k / 2 * 8 + n].x) = (float)(std::sqrt(2.0 / 8) * std::cos(pi * (2 * n + 1) * (2 * k + 1) / 32.0));
       d2[k * 8 + n] = (float)(std::sqrt(2.0 / 8) * std::cos(pi * k * (2 * n + 1) / 16.0));
     }
   for (int i = 0; i < 8; i++) hw[i] = (float)std::sin(pi / 16.0 * (i + 0.5));
-  cudaError_t e = cudaMemcpyToSymbol(c_dct4, d4, sizeof(d4));
+  cudaError_t e = cudaMemcpyToSymbol(c_dct4p, d4, sizeof(d4));
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_dct2e, d2, sizeof(d2));
   if (e == cudaSuccess) e = cudaMemcpyToSymbol(c_hwin, hw, sizeof(hw));
   return e;
@@ -46,13 +47,15 @@ cudaError_t upload_kernel_constants() {
 // ---------------------------------------------------------------------------
 // 8-point transforms on one lane's registers
 // ---------------------------------------------------------------------------
+// two outputs per packed multiply-add
 __device__ __forceinline__ void dct4_mat(const float x[8], float y[8]) {
 #pragma unroll
-  for (int k = 0; k < 8; k++) {
-    float s = 0.f;
+  for (int k = 0; k < 8; k += 2) {
+    float2 s = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int n = 0; n < 8; n++) s = fmaf(c_dct4[k * 8 + n], x[n], s);
-    y[k] = s;
+    for (int n = 0; n < 8; n++) s = __ffma2_rn(c_dct4p[k * 4 + n], make_float2(x[n], x[n]), s);
+    y[k] = s.x;
+    y[k + 1] = s.y;
   }
 }
 // DCT-IV, or DST-IV when `sine`: DST-IV(x)[k] = (-1)^k DCT-IV(reverse(x))[k]
@@ -99,11 +102,6 @@ __device__ __forceinline__ FoldIdx fold_idx(int x) {
   return f;
 }
 
-__device__ __forceinline__ int bayer_color(int x, int y, int rr, int rc) {
-  int xo = (x & 1) == rc, yo = (y & 1) == rr;
-  return (xo && yo) ? 0 : ((!xo && !yo) ? 1 : 2);
-}
-
 __device__ __forceinline__ int mirror(int p, int n) {  // ImageDtt.java:4958-4969
   if (p < 0) return p & 1;
   if (p >= n) return n - 2 + (p & 1);
@@ -120,131 +118,240 @@ __device__ __forceinline__ float warp_sum(float v) {
 // Stage 2: convert + correct, one warp per (task, sensor, colour)
 // ---------------------------------------------------------------------------
 #define CC_WARPS 4
+#define CC_MINB 4  // CTAs an SM
 #define WIN_STRIDE 17
+#define HALF_STRIDE 9  // a mosaic colour's window: 8 columns a row
 #define QBUF 288  // 4 quadrants x 8 rows x 9
 
-__device__ __forceinline__ void convert_correct_subtile(const SceneDev &sc, int task, int s, int c,
-                                                        float *wb, float *tb, int lane, float out_regs[4][2]) {
-  const int S = sc.num_sensors, C = sc.num_colors;
-  const SubtilePlan p = sc.plan[((size_t)task * S + s) * C + c];
-  // 1. 16x16 window (mirrored at the image border), one colour of the mosaic
-  {
-    const int W = sc.width, H = sc.height;
-    int col = lane & 15, r0 = lane >> 4;
-    int x = mirror(p.tlx + col, W);
-    const float scale = sc.color_scale[c];
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-      int row = 2 * k + r0;
-      int y = mirror(p.tly + row, H);
-      size_t o = (size_t)y * sc.img_pitch + x;
-      float v = (sc.img_dtype[s] == 1) ? (float)__ldg((const uint16_t *)sc.images[s] + o)
-                                    : __ldg((const float *)sc.images[s] + o);
-      if (C == 3) v = (bayer_color(x, y, sc.bayer_red_row, sc.bayer_red_col) == c) ? v * scale : 0.f;
-      else v *= scale;
-      wb[row * WIN_STRIDE + col] = v;
-    }
-  }
-  __syncwarp();
-  const int m = lane >> 3, r = lane & 7;
-  // 2. shifted-window fold (DttRad2.get_shifted_fold_2d + fold_tile), row r of quadrant m
-  float ahs, ahc, avs, avc;
-  sincospif(p.rx * 0.0625f, &ahs, &ahc);
-  sincospif(p.ry * 0.0625f, &avs, &avc);
-  float y[8];
-  {
-    FoldIdx fv = fold_idx(r);
-    float vw0 = avc * c_hwin[fv.win0] + avs * c_hwin[fv.dwin0] * fv.ds0;
-    float vw1 = avc * c_hwin[fv.win1] + avs * c_hwin[fv.dwin1] * fv.ds1;
-    bool vb = (m >> 1) & 1, hb = m & 1;
-    float vk0 = (vb ? fv.ss0 : fv.sc0) * vw0;
-    float vk1 = (vb ? fv.ss1 : fv.sc1) * vw1;
-    const float *row0 = wb + fv.src0 * WIN_STRIDE, *row1 = wb + fv.src1 * WIN_STRIDE;
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      FoldIdx fh = fold_idx(j);  // compile-time after unrolling
-      float hw0 = ahc * c_hwin[fh.win0] + ahs * c_hwin[fh.dwin0] * fh.ds0;
-      float hw1 = ahc * c_hwin[fh.win1] + ahs * c_hwin[fh.dwin1] * fh.ds1;
-      float hk0 = (hb ? fh.ss0 : fh.sc0) * hw0;
-      float hk1 = (hb ? fh.ss1 : fh.sc1) * hw1;
-      float a = fmaf(row0[fh.src1], hk1, row0[fh.src0] * hk0);
-      float b = fmaf(row1[fh.src1], hk1, row1[fh.src0] * hk0);
-      y[j] = fmaf(vk1, b, vk0 * a);
-    }
-  }
-  // 3. horizontal DCT-IV / DST-IV, transposed store (DttRad2.dttt_iv first pass)
-  float z[8];
-  dtt4(y, z, m & 1);
-#pragma unroll
-  for (int j = 0; j < 8; j++) tb[m * 72 + j * 9 + r] = z[j];
-  __syncwarp();
-#pragma unroll
-  for (int i = 0; i < 8; i++) y[i] = tb[m * 72 + r * 9 + i];
-  // 4. vertical DCT-IV / DST-IV: lane (m, r) now holds clt[m][r*8 + k], r = horizontal frequency
-  dtt4(y, z, (m >> 1) & 1);
-  __syncwarp();  // everyone done reading the window before it is reused
-#pragma unroll
-  for (int k = 0; k < 8; k++) wb[m * 72 + r * 9 + k] = z[k];
-  // shift coefficients: lanes 0-7 horizontal frequency i, lanes 8-15 vertical frequency k
-  float cs_s, cs_c;
-  {
-    int f = lane & 7;
-    float sh = (lane < 8) ? p.rx : p.ry;
-    sincospif((f + 0.5f) * sh * 0.125f, &cs_s, &cs_c);
-  }
-  __syncwarp();
-  // 5. CLT-domain convolution (ImageDtt.convolve_tile) and phase-rotation shift (fract_shift)
-  const float *kp = (p.kidx >= 0) ? sc.kernels[s] + (size_t)p.kidx * TP_CLT : nullptr;
-#pragma unroll
-  for (int h = 0; h < 2; h++) {
-    int idx = lane + 32 * h;
-    int off = (idx >> 3) * 9 + (idx & 7);
-    float d0 = wb[off], d1 = wb[72 + off], d2 = wb[144 + off], d3 = wb[216 + off];
-    float r0v = d0, r1v = d1, r2v = d2, r3v = d3;
-    if (kp) {
-      float k0 = __ldg(kp + idx), k1 = __ldg(kp + 64 + idx), k2 = __ldg(kp + 128 + idx), k3 = __ldg(kp + 192 + idx);
-      // zi = {{0,-1,-2,3},{1,0,-3,-2},{2,-3,0,-1},{3,2,1,0}} (ImageDtt.java:5458-5462)
-      r0v = d0 * k0 - d1 * k1 - d2 * k2 + d3 * k3;
-      r1v = d1 * k0 + d0 * k1 - d3 * k2 - d2 * k3;
-      r2v = d2 * k0 - d3 * k1 + d0 * k2 - d1 * k3;
-      r3v = d3 * k0 + d2 * k1 + d1 * k2 + d0 * k3;
-    }
-    int fi = idx >> 3, fk = idx & 7;
-    float ch = __shfl_sync(0xffffffffu, cs_c, fi), sh = __shfl_sync(0xffffffffu, cs_s, fi);
-    float cv = __shfl_sync(0xffffffffu, cs_c, 8 + fk), sv = __shfl_sync(0xffffffffu, cs_s, 8 + fk);
-    float t0 = r0v * ch - r1v * sh, t1 = r1v * ch + r0v * sh;
-    float t2 = r2v * ch - r3v * sh, t3 = r3v * ch + r2v * sh;
-    out_regs[0][h] = t0 * cv - t2 * sv;
-    out_regs[2][h] = t2 * cv + t0 * sv;
-    out_regs[1][h] = t1 * cv - t3 * sv;
-    out_regs[3][h] = t3 * cv + t1 * sv;
-  }
-  __syncwarp();
+__device__ __forceinline__ float window_pixel(const SceneDev &sc, int s, int x, int y) {
+  const size_t o = (size_t)mirror(y, sc.height) * sc.img_pitch + mirror(x, sc.width);
+  return (sc.img_dtype[s] == 1) ? (float)__ldg((const uint16_t *)sc.images[s] + o) : __ldg((const float *)sc.images[s] + o);
 }
 
-__global__ void __launch_bounds__(CC_WARPS * 32) convert_correct_kernel(SceneDev sc) {
+// Row r of quadrant m of the folded window: per value two source rows and two source columns, weighted by the
+// shifted window.  Of a mosaic colour's window one of the four products (red, blue) or one a row (green) is not zero,
+// and only those are formed.
+struct FoldRow {
+  FoldIdx f;
+  float vk0, vk1, ahs, ahc;
+};
+__device__ __forceinline__ FoldRow fold_row(float sn, float cs, int m, int r) {
+  FoldRow w;
+  w.ahs = __shfl_sync(0xffffffffu, sn, 16);
+  w.ahc = __shfl_sync(0xffffffffu, cs, 16);
+  const float avs = __shfl_sync(0xffffffffu, sn, 17), avc = __shfl_sync(0xffffffffu, cs, 17);
+  w.f = fold_idx(r);
+  const float vw0 = avc * c_hwin[w.f.win0] + avs * c_hwin[w.f.dwin0] * w.f.ds0;
+  const float vw1 = avc * c_hwin[w.f.win1] + avs * c_hwin[w.f.dwin1] * w.f.ds1;
+  const bool vb = (m >> 1) & 1;
+  w.vk0 = (vb ? w.f.ss0 : w.f.sc0) * vw0;
+  w.vk1 = (vb ? w.f.ss1 : w.f.sc1) * vw1;
+  return w;
+}
+__device__ __forceinline__ float fold_col0(const FoldRow &w, const FoldIdx &fh, bool hb) {
+  const float hw0 = w.ahc * c_hwin[fh.win0] + w.ahs * c_hwin[fh.dwin0] * fh.ds0;
+  return (hb ? fh.ss0 : fh.sc0) * hw0;
+}
+__device__ __forceinline__ float fold_col1(const FoldRow &w, const FoldIdx &fh, bool hb) {
+  const float hw1 = w.ahc * c_hwin[fh.win1] + w.ahs * c_hwin[fh.dwin1] * fh.ds1;
+  return (hb ? fh.ss1 : fh.sc1) * hw1;
+}
+__device__ __forceinline__ void fold_dense(const float *wb, float sn, float cs, int m, int r, float y[8]) {
+  const FoldRow w = fold_row(sn, cs, m, r);
+  const float *row0 = wb + w.f.src0 * WIN_STRIDE, *row1 = wb + w.f.src1 * WIN_STRIDE;
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    const FoldIdx fh = fold_idx(j);  // compile-time after unrolling
+    const float hk0 = fold_col0(w, fh, m & 1), hk1 = fold_col1(w, fh, m & 1);
+    const float a = fmaf(row0[fh.src1], hk1, row0[fh.src0] * hk0);
+    const float b = fmaf(row1[fh.src1], hk1, row1[fh.src0] * hk0);
+    y[j] = fmaf(w.vk1, b, w.vk0 * a);
+  }
+}
+// red or blue: rows of parity pr and columns of parity PC, [8][HALF_STRIDE]
+template <int PC>
+__device__ __forceinline__ void fold_one(const float *wb, float sn, float cs, int m, int r, int pr, float y[8]) {
+  const FoldRow w = fold_row(sn, cs, m, r);
+  const bool one = (w.f.src0 & 1) != pr;
+  const float *row = wb + ((one ? w.f.src1 : w.f.src0) >> 1) * HALF_STRIDE;
+  const float vk = one ? w.vk1 : w.vk0;
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    const FoldIdx fh = fold_idx(j);
+    const bool h1 = (fh.src0 & 1) != PC;  // known at compile time
+    y[j] = vk * (row[(h1 ? fh.src1 : fh.src0) >> 1] * (h1 ? fold_col1(w, fh, m & 1) : fold_col0(w, fh, m & 1)));
+  }
+}
+// green: of each row the columns with (row + column) of parity pg, [16][HALF_STRIDE]
+__device__ __forceinline__ void fold_two(const float *wb, float sn, float cs, int m, int r, int pg, float y[8]) {
+  const FoldRow w = fold_row(sn, cs, m, r);
+  const float *row0 = wb + w.f.src0 * HALF_STRIDE, *row1 = wb + w.f.src1 * HALF_STRIDE;
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    const FoldIdx fh = fold_idx(j);
+    const float hk0 = fold_col0(w, fh, m & 1), hk1 = fold_col1(w, fh, m & 1);
+    const bool a1 = ((fh.src0 + w.f.src0) & 1) != pg, b1 = ((fh.src0 + w.f.src1) & 1) != pg;
+    const float a = row0[(a1 ? fh.src1 : fh.src0) >> 1] * (a1 ? hk1 : hk0);
+    const float b = row1[(b1 ? fh.src1 : fh.src0) >> 1] * (b1 ? hk1 : hk0);
+    y[j] = fmaf(w.vk1, b, w.vk0 * a);
+  }
+}
+
+// An item of work: the subtile of one (task, sensor, colour)
+struct Subtile {
+  int task, s, c;
+  SubtilePlan p;
+};
+__device__ __forceinline__ Subtile subtile_of(const SceneDev &sc, int i) {
+  const int SC = sc.num_sensors * sc.num_colors;
+  Subtile t;
+  t.task = i / SC;
+  const int rem = i - t.task * SC;
+  t.s = rem / sc.num_colors;
+  t.c = rem - t.s * sc.num_colors;
+  t.p = sc.plan[(size_t)t.task * SC + rem];
+  return t;
+}
+// parities of a mosaic colour's pixels within the window: of the columns and rows (red, blue), of their sum (green)
+struct MosaicParity {
+  int pc, pr, pg;
+};
+__device__ __forceinline__ MosaicParity mosaic_parity(const SceneDev &sc, const Subtile &t) {
+  const int rr = sc.bayer_red_row, rc = sc.bayer_red_col;
+  return {((t.c == 0 ? rc : 1 - rc) - t.p.tlx) & 1, ((t.c == 0 ? rr : 1 - rr) - t.p.tly) & 1,
+          (t.p.tlx + t.p.tly + rc + rr + 1) & 1};
+}
+
+// A lane's pixels of a subtile's 16x16 window (mirrored at the image border, which keeps parities: width and height
+// are even): a red or blue window holds 64, a green one 128, a mono one 256.
+template <int C>
+__device__ __forceinline__ void window_load(const SceneDev &sc, const Subtile &t, int lane, float v[C == 3 ? 4 : 8]) {
+  const int m = lane >> 3, r = lane & 7;
+  if (C == 3) {
+    const MosaicParity mp = mosaic_parity(sc, t);
+    if (t.c < 2) {
+#pragma unroll
+      for (int k = 0; k < 2; k++)
+        v[k] = window_pixel(sc, t.s, t.p.tlx + 2 * r + mp.pc, t.p.tly + 2 * (4 * k + m) + mp.pr);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        v[k] = window_pixel(sc, t.s, t.p.tlx + 2 * r + ((m + mp.pg) & 1), t.p.tly + 4 * k + m);
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = window_pixel(sc, t.s, t.p.tlx + (lane & 15), t.p.tly + 2 * k + (lane >> 4));
+  }
+}
+
+// The window to shared memory and folded (DttRad2.get_shifted_fold_2d + fold_tile): row r of quadrant m
+template <int C>
+__device__ __forceinline__ void window_fold(const SceneDev &sc, const Subtile &t, float *wb, float sn, float cs, int lane,
+                                            const float v[C == 3 ? 4 : 8], float y[8]) {
+  const int m = lane >> 3, r = lane & 7;
+  const float scale = sc.color_scale[t.c];
+  if (C == 3) {
+    const MosaicParity mp = mosaic_parity(sc, t);
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (k < 2 || t.c == 2) wb[(4 * k + m) * HALF_STRIDE + r] = v[k] * scale;
+    __syncwarp();
+    if (t.c == 2) fold_two(wb, sn, cs, m, r, mp.pg, y);
+    else if (mp.pc) fold_one<1>(wb, sn, cs, m, r, mp.pr, y);
+    else fold_one<0>(wb, sn, cs, m, r, mp.pr, y);
+  } else {
+#pragma unroll
+    for (int k = 0; k < 8; k++) wb[(2 * k + (lane >> 4)) * WIN_STRIDE + (lane & 15)] = v[k] * scale;
+    __syncwarp();
+    fold_dense(wb, sn, cs, m, r, y);
+  }
+}
+
+// One warp per subtile, the next one's plan and pixels fetched meanwhile.  A mosaic window's other colours are
+// neither loaded nor multiplied (two to four loads a lane instead of eight), one sincospi serves a subtile.
+// 4 x 640x480 with kernel tables, 57,600 subtiles: 67 us with dense windows, 53 without the other colours and
+// 47 with the next subtile's loads ahead.  16 warps an SM at 128 registers: the transforms' 64 coefficients stay in
+// them; bounded to 96 or 80 the kernel spills (60 and 69 us).
+template <int C>
+__global__ void __launch_bounds__(CC_WARPS * 32, CC_MINB) convert_correct_kernel(const __grid_constant__ SceneDev sc) {
   __shared__ float smem[CC_WARPS][2 * QBUF];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, m = lane >> 3, r = lane & 7;
   float *wb = smem[warp];
   float *tb = wb + QBUF;  // window (16x17) and the CLT buffer (4x8x9) share the first QBUF floats
-  const int S = sc.num_sensors, C = sc.num_colors;
-  const int total = sc.num_tasks * S * C;
-  for (int st = blockIdx.x * CC_WARPS + warp; st < total; st += gridDim.x * CC_WARPS) {
-    int task = st / (S * C), rem = st - task * S * C;
-    int s = rem / C, c = rem - s * C;
-    float o[4][2];
-    convert_correct_subtile(sc, task, s, c, wb, tb, lane, o);
-    int txy = sc.task_txy[task];
-    size_t tile = (size_t)(txy >> 16) * sc.tilesX + (txy & 0xffff);
-    float *dst = sc.clt + ((tile * S + s) * C + c) * TP_CLT;
-    // the reference GPU's lpf_mask (TileProcessor.cuh:1037-1061): the stored CLT times the LPF
-    const bool lp = sc.lpf_rbg && ((sc.clt_lpf_mask >> c) & 1);
-    const float l0 = lp ? sc.lpf_rbg[c * 64 + lane] : 1.f, l1 = lp ? sc.lpf_rbg[c * 64 + lane + 32] : 1.f;
+  const int total = sc.num_tasks * sc.num_sensors * C, stride = gridDim.x * CC_WARPS;
+  int i = blockIdx.x * CC_WARPS + warp;
+  if (i >= total) return;  // whole warps
+  Subtile t = subtile_of(sc, i);
+  float v[C == 3 ? 4 : 8];
+  window_load<C>(sc, t, lane, v);
+  for (; i < total; i += stride) {
+    const bool more = i + stride < total;
+    const Subtile next = more ? subtile_of(sc, i + stride) : t;
+    const SubtilePlan p = t.p;
+    const float *kp = (p.kidx >= 0) ? sc.kernels[t.s] + (size_t)p.kidx * TP_CLT : nullptr;
+    float kk[4][2];
+    if (kp) {
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      dst[q * 64 + lane] = o[q][0] * l0;
-      dst[q * 64 + lane + 32] = o[q][1] * l1;
+      for (int q = 0; q < 4; q++) {
+        kk[q][0] = __ldg(kp + q * 64 + lane);
+        kk[q][1] = __ldg(kp + q * 64 + lane + 32);
+      }
     }
+    const int txy = sc.task_txy[t.task];
+    // 1. sines and cosines of the shift: lanes 0-7 horizontal frequency i, lanes 8-15 vertical frequency k (the
+    // phase rotation), lane 16 the horizontal and the other lanes the vertical shift (the window)
+    float sn, cs;
+    sincospif(lane < 16 ? (r + 0.5f) * (lane < 8 ? p.rx : p.ry) * 0.125f : (lane == 16 ? p.rx : p.ry) * 0.0625f, &sn, &cs);
+    // 2. one colour's window, folded
+    float y[8];
+    window_fold<C>(sc, t, wb, sn, cs, lane, v, y);
+    if (more) window_load<C>(sc, next, lane, v);
+    // 3. horizontal DCT-IV / DST-IV, transposed store (DttRad2.dttt_iv first pass)
+    float z[8];
+    dtt4(y, z, m & 1);
+#pragma unroll
+    for (int j = 0; j < 8; j++) tb[m * 72 + j * 9 + r] = z[j];
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 8; j++) y[j] = tb[m * 72 + r * 9 + j];
+    // 4. vertical DCT-IV / DST-IV: lane (m, r) now holds clt[m][r*8 + k], r = horizontal frequency
+    dtt4(y, z, (m >> 1) & 1);
+    __syncwarp();  // everyone done reading the window before it is reused
+#pragma unroll
+    for (int k = 0; k < 8; k++) wb[m * 72 + r * 9 + k] = z[k];
+    __syncwarp();
+    // 5. CLT-domain convolution (ImageDtt.convolve_tile) and phase-rotation shift (fract_shift), on CLT indices
+    // lane and lane + 32
+    const size_t tile = (size_t)(txy >> 16) * sc.tilesX + (txy & 0xffff);
+    float *dst = sc.clt + ((tile * sc.num_sensors + t.s) * C + t.c) * TP_CLT;
+    // the reference GPU's lpf_mask (TileProcessor.cuh:1037-1061): the stored CLT times the LPF
+    const bool lp = sc.lpf_rbg && ((sc.clt_lpf_mask >> t.c) & 1);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int idx = lane + 32 * h, off = (idx >> 3) * 9 + (idx & 7);
+      float d0 = wb[off], d1 = wb[72 + off], d2 = wb[144 + off], d3 = wb[216 + off];
+      float r0v = d0, r1v = d1, r2v = d2, r3v = d3;
+      if (kp) {
+        const float k0 = kk[0][h], k1 = kk[1][h], k2 = kk[2][h], k3 = kk[3][h];
+        // zi = {{0,-1,-2,3},{1,0,-3,-2},{2,-3,0,-1},{3,2,1,0}} (ImageDtt.java:5458-5462)
+        r0v = d0 * k0 - d1 * k1 - d2 * k2 + d3 * k3;
+        r1v = d1 * k0 + d0 * k1 - d3 * k2 - d2 * k3;
+        r2v = d2 * k0 - d3 * k1 + d0 * k2 - d1 * k3;
+        r3v = d3 * k0 + d2 * k1 + d1 * k2 + d0 * k3;
+      }
+      const int fi = idx >> 3, fk = idx & 7;
+      const float ch = __shfl_sync(0xffffffffu, cs, fi), sh = __shfl_sync(0xffffffffu, sn, fi);
+      const float cv = __shfl_sync(0xffffffffu, cs, 8 + fk), sv = __shfl_sync(0xffffffffu, sn, 8 + fk);
+      const float t0 = r0v * ch - r1v * sh, t1 = r1v * ch + r0v * sh;
+      const float t2 = r2v * ch - r3v * sh, t3 = r3v * ch + r2v * sh;
+      const float l = lp ? sc.lpf_rbg[t.c * 64 + idx] : 1.f;
+      dst[idx] = (t0 * cv - t2 * sv) * l;
+      dst[64 + idx] = (t1 * cv - t3 * sv) * l;
+      dst[128 + idx] = (t2 * cv + t0 * sv) * l;
+      dst[192 + idx] = (t3 * cv + t1 * sv) * l;
+    }
+    __syncwarp();
+    t = next;
   }
 }
 
@@ -656,7 +763,8 @@ static int grid_for(int items, int per_block) {
 cudaError_t launch_convert_correct(const SceneDev &sc, cudaStream_t st) {
   int n = sc.num_tasks * sc.num_sensors * sc.num_colors;
   if (n <= 0) return cudaSuccess;
-  convert_correct_kernel<<<grid_for(n, CC_WARPS), CC_WARPS * 32, 0, st>>>(sc);
+  if (sc.num_colors == 3) convert_correct_kernel<3><<<grid_for(n, CC_WARPS), CC_WARPS * 32, 0, st>>>(sc);
+  else convert_correct_kernel<1><<<grid_for(n, CC_WARPS), CC_WARPS * 32, 0, st>>>(sc);
   return cudaGetLastError();
 }
 
