@@ -25,6 +25,7 @@
 //  phase C  one warp = one tile: combine the per-warp strip products, integer
 //           argmax on the disparity axis, windowed centroid, hor/vert maxima.
 #include "tp_forward.cuh"
+#include "tp_pairs.cuh"
 #include "tp_launch.h"
 
 // ---------------------------------------------------------------------------
@@ -547,28 +548,65 @@ cudaError_t launch_rig(const SceneDev &mn, const SceneDev &ax, const CorrConst &
 
 // ---------------------------------------------------------------------------
 // IMCLT (ImageDtt.iclt_2d, the reference GPU imclt_rbg) with overlap-add into the
-// padded colour frames.  CTA = one 64x64-pixel region of one (sensor, colour)
-// plane; the 9x9 tiles touching it are processed in the four tile-parity phases
+// padded colour frames.  CTA = one region of IR x IR blocks of 8x8 pixels of one (sensor, colour)
+// plane; the (IR + 1)^2 tiles touching it are processed in the four tile-parity phases
 // (tiles of one phase never overlap), so the region accumulates in shared memory
 // without atomics and in a fixed order.  A warp carries 4 tiles at once, one per
-// 8-lane group, lane r owning row r of each quadrant.
+// 8-lane group, lane r owning row r of each quadrant; the transforms carry quadrants m and m + 2
+// two values per instruction.
+// 12 planes of 1296x968 and of 640x480: 113 and 38.6 us with scalar transforms, 14 x 14 blocks and nine warps, 108
+// and 33.7 with these; 12 and seven 107 and 32.6, 10 and five 105 and 30.7, 8 and seven 116 and 32.0.  What bounds
+// it: the phases' barriers and the latency of each phase's first loads.
 // ---------------------------------------------------------------------------
-constexpr int IMCLT_IR = 14;     // region = IR x IR blocks of 8x8 pixels (14: 0.41 ms, 16: 0.43, 12: 0.44 on 4x2592x1936)
-constexpr int IMCLT_WARPS = 9;   // 36 8-lane groups: the four parity phases (49, 56, 56, 64 tiles) in 2 rounds each
+// dct4_fast (tp_dtt.cuh) of two rows, the same operations
+__device__ __forceinline__ void dct4_two(const float2 x[8], float2 y[8]) {
+  const float2 C18 = dup2(1.3065629648763766f), C38 = dup2(0.5411961001461970f), N18 = dup2(-1.3065629648763766f),
+               SQ2 = dup2(1.4142135623730951f);
+  float2 u0[4], u1[4], v0[4], v1[4];
+#pragma unroll
+  for (int j = 0; j < 4; j++) {
+    u0[j] = fma2(dup2(k_d4c[j]), x[j], mul2(dup2(k_d4s[j]), x[7 - j]));
+    // the odd ones negated in their factors
+    const float sg = (j & 1) ? -1.f : 1.f;
+    u1[j] = fma2(dup2(sg * k_d4c[3 - j]), x[4 + j], mul2(dup2(-sg * k_d4s[3 - j]), x[3 - j]));
+  }
+  {
+    const float2 a0 = add2(u0[0], u0[3]), a1 = add2(u0[1], u0[2]), b0 = sub2(u0[0], u0[3]), b1 = sub2(u0[1], u0[2]);
+    v0[0] = add2(a0, a1); v0[2] = sub2(a0, a1);
+    v0[1] = fma2(C18, b0, mul2(C38, b1)); v0[3] = fma2(C38, b0, mul2(N18, b1));
+  }
+  {
+    const float2 a0 = add2(u1[0], u1[3]), a1 = add2(u1[1], u1[2]), b0 = sub2(u1[0], u1[3]), b1 = sub2(u1[1], u1[2]);
+    v1[0] = add2(a0, a1); v1[2] = sub2(a0, a1);
+    v1[1] = fma2(C18, b0, mul2(C38, b1)); v1[3] = fma2(C38, b0, mul2(N18, b1));
+  }
+  y[0] = mul2(SQ2, v0[0]);
+  y[7] = mul2(SQ2, v1[0]);
+  y[2] = add2(v0[1], v1[3]);
+  y[4] = sub2(v0[2], v1[2]);
+  y[6] = add2(v0[3], v1[1]);
+  y[1] = sub2(v0[1], v1[3]);
+  y[3] = add2(v0[2], v1[2]);
+  y[5] = sub2(v0[3], v1[1]);
+}
 
-template <int IR>
-__global__ void __launch_bounds__(32 * IMCLT_WARPS) imclt_fast_kernel(const __grid_constant__ SceneDev sc) {
+constexpr int IMCLT_IR = 10;      // region = IR x IR blocks of 8x8 pixels
+constexpr int IMCLT_WARPS = 5;    // the four parity phases (25, 30, 30, 36 tiles), four tiles a warp, in two rounds each
+constexpr int IMCLT_SMALL = 152;  // regions for a region on each SM
+
+template <int IR, int NW>
+__global__ void __launch_bounds__(32 * NW) imclt_fast_kernel(const __grid_constant__ SceneDev sc) {
   constexpr int IPX = IR * 8, ISTR = IPX + 1;
   extern __shared__ float acc[];  // [IPX][ISTR]
-  __shared__ float tbuf_all[IMCLT_WARPS][4 * 72];
+  __shared__ float2 tbuf_all[NW][4 * 72];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = lane >> 3, r = lane & 7;
   const int S = sc.num_sensors, C = sc.num_colors;
   const int plane = blockIdx.z, s = plane / C, c = plane - s * C;
   const int bx0 = blockIdx.x * IR, by0 = blockIdx.y * IR;
   const int fw = sc.width + 8, fh = sc.height + 8;
-  for (int i = threadIdx.x; i < IPX * ISTR; i += blockDim.x) acc[i] = 0.f;
+  for (int i = threadIdx.x; i < IPX * ISTR; i += 32 * NW) acc[i] = 0.f;
   __syncthreads();
-  float *tbuf = tbuf_all[warp] + q * 72;
+  float2 *tbuf = tbuf_all[warp] + q * 72;
   // (a stored CLT that already carries the LPF, clt_lpf_mask, is not filtered again)
   const float *lpf = (sc.lpf_rbg && !((sc.clt_lpf_mask >> c) & 1)) ? sc.lpf_rbg + c * 64 : nullptr;
   // unfold rows fed by source row r (DttRad2.get_unfold_index_signs, 392-404)
@@ -576,84 +614,102 @@ __global__ void __launch_bounds__(32 * IMCLT_WARPS) imclt_fast_kernel(const __gr
   const float sa1 = (r >= 4) ? 1.f : -1.f, sb1 = 1.f;    // signs (cos, sin branch) of row i1
   const float sa2 = -1.f, sb2 = (r >= 4) ? 1.f : -1.f;   // signs of row i2
   const float w1 = k_hwin[i1 < 8 ? i1 : 15 - i1], w2 = k_hwin[i2 < 8 ? i2 : 15 - i2];
-  const float kc1 = sa1 * w1, ks1 = sb1 * w1, kc2 = sa2 * w2, ks2 = sb2 * w2;
+  // the DST-IV of quadrants 2 and 3 in the first pass leaves the odd rows negative: sg
+  const float sg = (r & 1) ? -1.f : 1.f;
+  const float kc1 = sa1 * w1, ks1 = sg * sb1 * w1, kc2 = sa2 * w2, ks2 = sg * sb2 * w2;
   float lk[8];  // 0.25 x the colour's LPF for row r (the iclt_2d scale)
 #pragma unroll
   for (int v = 0; v < 8; v++) lk[v] = 0.25f * (lpf ? lpf[r * 8 + v] : 1.0f);
+#pragma unroll 1
   for (int ph = 0; ph < 4; ph++) {
     const int pxp = ph & 1, pyp = ph >> 1;
     int tx0 = bx0 - 1, ty0 = by0 - 1;
     if ((tx0 & 1) != pxp) tx0++;
     if ((ty0 & 1) != pyp) ty0++;
     const int ntx = (bx0 + IR - 1 - tx0) / 2 + 1, nty = (by0 + IR - 1 - ty0) / 2 + 1;
-    for (int k0 = warp * 4; k0 < ntx * nty; k0 += 4 * IMCLT_WARPS) {
+#pragma unroll 1
+    for (int k0 = warp * 4; k0 < ntx * nty; k0 += 4 * NW) {
       const int k = k0 + q;
       const int tx = tx0 + 2 * (k % ntx), ty = ty0 + 2 * (k / ntx);
       bool act = k < ntx * nty && tx >= 0 && ty >= 0 && tx < sc.tilesX && ty < sc.tilesY;
-      size_t tile = act ? (size_t)ty * sc.tilesX + tx : 0;
+      const size_t tile = act ? (size_t)ty * sc.tilesX + tx : 0;
       if (act && sc.tile_task[tile] < 0) act = false;
-      float o[4][8];
       const float *src = sc.clt + ((tile * S + s) * C + c) * TP_CLT + r * 8;
+      // inverse 2D DCT-IV/DST-IV with the swapped mode (ImageDtt.java:3628): rows (vertical frequency) first,
+      // then columns; DST-IV(x)[k] = (-1)^k DCT-IV(reversed x)[k]
+      float2 p[2][8];  // quadrants (0, 2) and (1, 3): vertical position r, horizontal positions
 #pragma unroll
-      for (int m = 0; m < 4; m++) {
-        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+      for (int m = 0; m < 2; m++) {
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a, d = a, e = a;
         if (act) {
           a = __ldg((const float4 *)(src + m * 64));
           b = __ldg((const float4 *)(src + m * 64 + 4));
+          d = __ldg((const float4 *)(src + m * 64 + 128));
+          e = __ldg((const float4 *)(src + m * 64 + 132));
         }
-        o[m][0] = a.x; o[m][1] = a.y; o[m][2] = a.z; o[m][3] = a.w;
-        o[m][4] = b.x; o[m][5] = b.y; o[m][6] = b.z; o[m][7] = b.w;
+        p[m][0] = make_float2(a.x * lk[0], e.w * lk[7]);
+        p[m][1] = make_float2(a.y * lk[1], e.z * lk[6]);
+        p[m][2] = make_float2(a.z * lk[2], e.y * lk[5]);
+        p[m][3] = make_float2(a.w * lk[3], e.x * lk[4]);
+        p[m][4] = make_float2(b.x * lk[4], d.w * lk[3]);
+        p[m][5] = make_float2(b.y * lk[5], d.z * lk[2]);
+        p[m][6] = make_float2(b.z * lk[6], d.y * lk[1]);
+        p[m][7] = make_float2(b.w * lk[7], d.x * lk[0]);
       }
 #pragma unroll
-      for (int v = 0; v < 8; v++)
+      for (int m = 0; m < 2; m++) {
+        float2 z[8];
+        dct4_two(p[m], z);
 #pragma unroll
-        for (int m = 0; m < 4; m++) o[m][v] *= lk[v];
-      // inverse 2D DCT-IV/DST-IV with the swapped mode (ImageDtt.java:3628):
-      // rows (vertical frequency) first, then columns
-      float t[4][8];
+        for (int j = 0; j < 8; j++) tbuf[j * 9 + r] = z[j];
+        __syncwarp();
 #pragma unroll
-      for (int m = 0; m < 4; m++) {
-        float z[8];
-        dtt4_fast(o[m], z, (m >> 1) & 1);
-        group_transpose(z, tbuf, r);
-        dtt4_fast(z, t[m], m & 1);  // lane r: vertical position r, t[m][x] horizontal position x
+        for (int j = 0; j < 8; j++) z[j] = tbuf[r * 9 + (m ? 7 - j : j)];
+        __syncwarp();
+        dct4_two(z, p[m]);  // quadrants 1 and 3: the odd positions are negative
       }
       // unfold (DttRad2.unfold_tile) into rows i1, i2 and accumulate
-      const int gy1 = ty * 8 + i1 - by0 * 8, gy2 = ty * 8 + i2 - by0 * 8;
+      const int gx0 = (tx - bx0) * 8, gy1 = (ty - by0) * 8 + i1, gy2 = (ty - by0) * 8 + i2;
+      const bool left = act && gx0 >= 0, right = act && gx0 + 8 < IPX;  // the tile's halves lie in the region
+      const bool r1 = gy1 >= 0 && gy1 < IPX, r2 = gy2 >= 0 && gy2 < IPX;
+      float *a1 = acc + gy1 * ISTR + gx0, *a2 = acc + gy2 * ISTR + gx0;
 #pragma unroll
       for (int jj = 0; jj < 16; jj++) {
         const int seg = jj >> 2, xx = jj & 3;
         const int ih = (seg == 0) ? xx + 4 : ((seg == 1) ? 7 - xx : ((seg == 2) ? 3 - xx : xx));
-        const float hs1 = (seg == 0) ? 1.f : -1.f, hs2 = (seg == 3) ? -1.f : 1.f;
+        const float hs1 = (seg == 0) ? 1.f : -1.f, hs2 = ((seg == 3) != ((ih & 1) != 0)) ? -1.f : 1.f;
         const float wh = k_hwin[jj < 8 ? jj : 15 - jj];
-        const float khc = hs1 * wh, khs = hs2 * wh;
-        const float A = fmaf(khs, t[1][ih], khc * t[0][ih]);
-        const float B = fmaf(khs, t[3][ih], khc * t[2][ih]);
-        const int gx = tx * 8 + jj - bx0 * 8;
-        if (act && gx >= 0 && gx < IPX) {
-          if (gy1 >= 0 && gy1 < IPX) acc[gy1 * ISTR + gx] += fmaf(ks1, B, kc1 * A);
-          if (gy2 >= 0 && gy2 < IPX) acc[gy2 * ISTR + gx] += fmaf(ks2, B, kc2 * A);
-        }
+        const float2 ab = fma2(dup2(hs2 * wh), p[1][ih], mul2(dup2(hs1 * wh), p[0][ih]));
+        const bool in = jj < 8 ? left : right;
+        if (in && r1) a1[jj] += fmaf(ks1, ab.y, kc1 * ab.x);
+        if (in && r2) a2[jj] += fmaf(ks2, ab.y, kc2 * ab.x);
       }
     }
     __syncthreads();
   }
-  float *dst = sc.rbg + (size_t)plane * fw * fh;
-  for (int i = threadIdx.x; i < IPX * IPX; i += blockDim.x) {
-    const int ly = i / IPX, lx = i - ly * IPX;
-    const int gx = bx0 * 8 + lx, gy = by0 * 8 + ly;
-    if (gx < fw && gy < fh) dst[(size_t)gy * fw + gx] = acc[ly * ISTR + lx];
+  float *dst = sc.rbg + (size_t)plane * fw * fh + bx0 * 8;
+  for (int ly = warp; ly < IPX && by0 * 8 + ly < fh; ly += NW) {
+    float *row = dst + (size_t)(by0 * 8 + ly) * fw;
+    for (int lx = lane; lx < IPX && bx0 * 8 + lx < fw; lx += 32) row[lx] = acc[ly * ISTR + lx];
   }
 }
 
-cudaError_t launch_imclt_fast(const SceneDev &sc, cudaStream_t st) {
-  constexpr int IR = IMCLT_IR;
+template <int IR, int NW>
+static cudaError_t go_imclt(const SceneDev &sc, cudaStream_t st) {
   const int bytes = IR * 8 * (IR * 8 + 1) * 4;
-  cudaError_t e = cudaFuncSetAttribute(imclt_fast_kernel<IR>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  const cudaError_t e = cudaFuncSetAttribute(imclt_fast_kernel<IR, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) return e;
-  dim3 grid((sc.tilesX + 1 + IR - 1) / IR, (sc.tilesY + 1 + IR - 1) / IR, sc.num_sensors * sc.num_colors);
-  imclt_fast_kernel<IR><<<grid, 32 * IMCLT_WARPS, bytes, st>>>(sc);
+  const dim3 grid((sc.tilesX + 1 + IR - 1) / IR, (sc.tilesY + 1 + IR - 1) / IR, sc.num_sensors * sc.num_colors);
+  imclt_fast_kernel<IR, NW><<<grid, 32 * NW, bytes, st>>>(sc);
   return cudaGetLastError();
+}
+
+cudaError_t launch_imclt_fast(const SceneDev &sc, cudaStream_t st) {
+  // Regions of 10 x 10 blocks need the fewest repeated tiles among the sizes with enough warps an SM; where they
+  // would leave SMs without one, 6 x 6 (four mono planes of 128x96: 14 us and 9 us; 12 planes of 1296x968: 105 us
+  // and 109 us).
+  const int regions = ((sc.tilesX + IMCLT_IR) / IMCLT_IR) * ((sc.tilesY + IMCLT_IR) / IMCLT_IR) * sc.num_sensors * sc.num_colors;
+  return regions < IMCLT_SMALL ? go_imclt<6, 4>(sc, st) : go_imclt<IMCLT_IR, IMCLT_WARPS>(sc, st);
 }
 
 __global__ void disp_init_kernel(float *disp, int n) {
