@@ -1398,8 +1398,13 @@ static tp_status batch_tables(tp_batch *b) {
     t += sc.num_tasks;
     const int c = batch_class(sc);
     // a warp-per-tile scene with at least 8 waves of tiles (16 warps per SM) has no tail
-    // worth sharing: it keeps its own launch, captured in the same graph
-    if (c != 2 && sc.num_tasks >= 8 * 16 * sms) {
+    // worth sharing: it keeps its own launch, captured in the same graph.  So does a many-pair scene that
+    // many_kernel takes (the queue runs the general pair split) from one wave of its six CTAs an SM on: eight
+    // scenes of 16 sensors and 120 pairs, own launch and queue: 5,120 tiles 3.1 and 4.0 ms, 1,920 1.24 and 1.51,
+    // 1,280 0.91 and 1.04, 320 0.42 and 0.32
+    const tp_handle *h = b->scenes[i];
+    const bool many = c == 2 && many_forward_ok(sc) && ((h->sched_tpb <= 0 && h->sched_nw <= 0) || (h->sched_tpb == 1 && h->sched_nw == 4));
+    if ((c != 2 && sc.num_tasks >= 8 * 16 * sms) || (many && sc.num_tasks >= 6 * sms)) {
       b->solo[c].push_back(b->scenes[i]);
       continue;
     }

@@ -105,3 +105,30 @@ def test_batch_matches_per_scene():
     finally:
         for tp in tps:
             tp.close()
+
+
+def test_many_pair_scenes_batch_with_and_without_own_launch():
+    """Many-pair scenes on both sides of the size from which they keep their own launch (1,920 and 320 tiles), as a
+    step and as a graph: the per-scene results, bit for bit where the launch is the per-scene one."""
+    sizes = [(384, 320), (160, 128), (384, 320)]
+    tps = []
+    try:
+        for i, (w, h) in enumerate(sizes):
+            sc = synth.make_scene("circle_lwir", seed=57 + i, width=w, height=h)
+            tps.append(_make(sc, None, None, synth.circle_pairs(sc["geometry"]), 2.0))
+        ref = []
+        for tp in tps:
+            tp.process()
+            ref.append(_results(tp))
+        with Batch(tps) as b:
+            for step in (lambda: b.process(replan=True), b.run_graph, b.run_graph):
+                step()
+                b.synchronize()
+                for i, (tp, r) in enumerate(zip(tps, ref)):
+                    got = _results(tp)
+                    _same(got, r)
+                    if i != 1:
+                        assert all(np.array_equal(x, y, equal_nan=True) for x, y in zip(got, r))
+    finally:
+        for tp in tps:
+            tp.close()
