@@ -1,5 +1,7 @@
 // tp_fused.cu -- fused forward tile kernel: convert+correct -> pair correlation
-// -> strip combination -> disparity extraction, one CTA per group of tiles.
+// -> strip combination -> disparity extraction, one CTA per group of tiles, for the scenes that
+// tp_quad.cu (standard quads) and tp_many.cu (many general pairs) do not take; the choice between
+// them (launch_fused_forward); the rig's inter-camera correlation; IMCLT.
 //
 // Same arithmetic as the stage kernels (ImageDtt.extract_correct_tile,
 // convolve_tile, fract_shift; Correlation2d.correlateCompositeFD,
