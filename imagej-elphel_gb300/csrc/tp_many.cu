@@ -9,7 +9,8 @@
 // pass of its own, where here three warps would wait for the fourth.
 // Results are the same bits: every warp's pairs are summed in the same order.
 // Measured on 16x640x512 (5,120 tiles): 500 -> 380 us; 480 warp instructions a pair (677 before), the
-// surfaces' 553 MB alone take 81 us.  What bounds it now: those chains, then the shared-memory pipe.
+// surfaces' 553 MB alone take 81 us; 375 with the windows 8 banks apart, 370 with a first sensor that both pairs
+// share (more than half of the couples) read once.  What bounds it now: the shared-memory pipe (78 %).
 #include "tp_forward.cuh"
 #include "tp_launch.h"
 #include "tp_pairs.cuh"
@@ -48,20 +49,29 @@ __device__ __forceinline__ float tap_strip(const float *c, float4 tap, int cells
   return out ? CUDART_NAN_F : (both ? 0.5f * d + 0.5f * d2 : d);
 }
 
-// the normalised, filtered spectra of two pairs into b (interleaved [4][8][9])
+// the normalised, filtered spectra of two pairs into b (interleaved [4][8][9]); the pairs are numbered by their first
+// sensor, which two that lie four apart mostly share
 __device__ __forceinline__ void couple_spectra(const CorrConst &cfg, const PairDev &pa, const PairDev &pb, float2 l0,
                                                float2 l1, const float *s_clt, float2 *b, int lane) {
   const float *a1 = s_clt + pa.cam1 * TP_CLT + lane, *a2 = s_clt + pa.cam2 * TP_CLT + lane;
   const float *b1 = s_clt + pb.cam1 * TP_CLT + lane, *b2 = s_clt + pb.cam2 * TP_CLT + lane;
   float2 d1[2][4], d2[2][4], amp[2];
 #pragma unroll
-  for (int h = 0; h < 2; h++) {
+  for (int h = 0; h < 2; h++)
 #pragma unroll
     for (int m = 0; m < 4; m++) {
       const int o = m * 64 + 32 * h;
-      d1[h][m] = make_float2(a1[o], b1[o]);
+      d1[h][m] = dup2(a1[o]);
       d2[h][m] = make_float2(a2[o], b2[o]);
     }
+  if (pa.cam1 != pb.cam1) {
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+      for (int m = 0; m < 4; m++) d1[h][m].y = b1[m * 64 + 32 * h];
+  }
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
     float2 s1 = mul2(d1[h][0], d1[h][0]), s2 = mul2(d2[h][0], d2[h][0]);
 #pragma unroll
     for (int m = 1; m < 4; m++) {
