@@ -239,11 +239,15 @@ __device__ __forceinline__ void shift_out(const SceneDev &sc, const SubtilePlan 
 // dd/d(port x, port y) of one (sensor, colour) sub-tile, 8-lane group: its dd/dCLT gl taken back to the folded
 // tile, which is dotted with the fold of the pixels under the derivative window, one fold per direction,
 // plus the rotation's own derivative.  gl is overwritten (with the folded gradient) where `own` is set.
-// ASYNC: w is a staged window whose copies are waited for before it is read.
-template <bool ASYNC = false, typename PIX>
+// stage() is called by the whole warp once clt is no longer needed: it may copy the windows over it,
+// asynchronously.
+struct NoStage {
+  __device__ __forceinline__ void operator()() const {}
+};
+template <typename PIX, typename STAGE = NoStage>
 __device__ __forceinline__ void shift_sens(const SceneDev &sc, const PIX &w, const SubtilePlan &p, int s,
                                            const float *clt, float *gl_all, float *tbq, int r, bool own,
-                                           float out[2]) {
+                                           float out[2], STAGE stage = STAGE()) {
   const float *kp = (p.kidx >= 0) ? sc.kernels[s] + (size_t)p.kidx * TP_CLT : nullptr;
   float ahs, ahc, avs, avc;
   __sincosf(CUDART_PI_F * 0.0625f * p.rx, &ahs, &ahc);
@@ -262,7 +266,9 @@ __device__ __forceinline__ void shift_sens(const SceneDev &sc, const PIX &w, con
       }
     }
   }
-  if (ASYNC) cp_async_wait_all();
+  __syncwarp();
+  stage();
+  cp_async_wait_all();
   __syncwarp();
   // the lane's two source rows of the window, read once for both directions and both vertical
   // variants

@@ -6,17 +6,19 @@
 // pairs on distinct sensors (16 sensors: 15 rounds of 8); the strip taps come from the forward's table;
 // and the windows of the shift derivatives are staged (tp_forward.cuh).
 // Needs the forward's strip samples (SceneDev::strips) and a strip of at most 32 entries.
-// Measured on 16x640x512 (5,120 tiles, 120 pairs): 992 -> 638 us.  What bounds it now: the shared-memory
-// pipe (about 65 %: the pairs' CLT reads and gradient updates are 96 of some 350 accesses a couple) and
-// the latency of those accesses at 16 warps an SM (32 KB of CLT and gradient a tile).
+// Measured on 16x640x512 (5,120 tiles, 120 pairs): 992 -> 640 us; 617 with the windows over a group's CLT once it is
+// read, which leaves room for a fifth CTA an SM (96 registers; with 128 and four CTAs 643).  What bounds it
+// now: the shared-memory pipe (about 70 %: the pairs' CLT reads and gradient updates are 96 of some 350 accesses a
+// couple) and the latency of those accesses at 20 warps an SM (32 KB of CLT and gradient a tile).
 #include "tp_adjoint_pairs.cuh"
 #include "tp_launch.h"
 
 namespace {
 
-constexpr int AM_WARP = 4 * Stage<false>::WIN;     // a warp's space: the gradients of its two pairs' surfaces, over them
-                                                   // the spectra; at the end its four windows
-static_assert(QP_BUF <= AM_WARP && 2 * AM_SURF <= AM_WARP, "a warp's space");
+constexpr int AM_WARP = QP_BUF;  // a warp's space: the gradients of its two pairs' surfaces, over them the spectra
+static_assert(2 * AM_SURF <= AM_WARP, "a warp's space");
+// at the end a group's windows: three over its CLT, the last one in the warp's space
+static_assert(3 * Stage<false>::WIN <= 4 * TP_CLT && Stage<false>::WIN <= AM_WARP, "a group's windows");
 __host__ __device__ constexpr int am_floats(int S) {  // CLT and its gradient, strip, the warps' space
   return ((S + 3) / 4) * 8 * TP_CLT + 64 + AD_NW * AM_WARP;
 }
@@ -38,7 +40,7 @@ __device__ __forceinline__ void scatter_strips(float *g, float f0, float f1, con
 }  // namespace
 
 template <bool U16>
-__global__ void __launch_bounds__(32 * AD_NW, 4) adjoint_many_kernel(const __grid_constant__ SceneDev sc,
+__global__ void __launch_bounds__(32 * AD_NW, 5) adjoint_many_kernel(const __grid_constant__ SceneDev sc,
                                                                      const __grid_constant__ CorrConst cfg, int RE,
                                                                      float *sens, float *dval) {
   extern __shared__ float sm[];
@@ -142,10 +144,9 @@ __global__ void __launch_bounds__(32 * AD_NW, 4) adjoint_many_kernel(const __gri
       const bool act = s < S;
       const int sidx = act ? s : S - 1;
       const SubtilePlan p = sc.plan[(size_t)task * S + sidx];
-      stage_window<U16>(sc, sc.images[sidx], p.tlx, p.tly, wb + q * Stage<U16>::WIN, r);
-      cp_async_commit();
+      float *wq = q < 3 ? s_clt + g * 4 * TP_CLT + q * Stage<U16>::WIN : wb;
       SWin<U16> win;
-      win.base = (const typename Stage<U16>::T *)(wb + q * Stage<U16>::WIN);
+      win.base = (const typename Stage<U16>::T *)wq;
       win.sx = p.tlx & (Stage<U16>::CH - 1);
       win.scale = sc.color_scale[0];
       // the group's transposes go through the sensor's CLT once it is read; a lane group beyond the last
@@ -159,8 +160,11 @@ __global__ void __launch_bounds__(32 * AD_NW, 4) adjoint_many_kernel(const __gri
       }
       __syncwarp();
       float gxy[2];
-      shift_sens<true>(sc, win, p, sidx, s_clt + (size_t)s * TP_CLT, s_g + (size_t)s * TP_CLT,
-                       s_clt + (size_t)s * TP_CLT, r, true, gxy);
+      shift_sens(sc, win, p, sidx, s_clt + (size_t)s * TP_CLT, s_g + (size_t)s * TP_CLT, s_clt + (size_t)s * TP_CLT, r,
+                 true, gxy, [&]() {
+                   stage_window<U16>(sc, sc.images[sidx], p.tlx, p.tly, wq, r);
+                   cp_async_commit();
+                 });
       if (r == 0 && act) {
         sens[(tile * S + s) * 2] = gxy[0];
         sens[(tile * S + s) * 2 + 1] = gxy[1];
