@@ -179,9 +179,9 @@ __global__ void __launch_bounds__(128, 4) fused_forward_win_kernel(const __grid_
 #pragma unroll
     for (int t = 0; t < NT; t++) {
       const int e = lane + 32 * t;
-      if (e < RE) sc.combo[tile * RE + e] = cmb[t];
+      if (e < RE) sc.sprod[(size_t)task * RE + e] = cmb[t];
     }
-    float4 *ob = (float4 *)(sc.osum + (tile * 32 + lane) * 8);
+    float4 *ob = (float4 *)(sc.osum + ((size_t)task * 32 + lane) * 8);
     ob[0] = make_float4(oprod[0], oprod[1], oprod[2], oprod[3]);
     ob[1] = make_float4(oprod[4], oprod[5], oprod[6], oprod[7]);
   }
@@ -847,7 +847,7 @@ cudaError_t launch_fused_forward(const SceneDev &sc, const CorrConst &cc, int tp
   for (int i = 0; i < sc.num_sensors; i++) all16 = all16 && sc.img_dtype[i] == 1;
   auto go = [&](auto kernel) { return launch_persistent(kernel, f.nw * 32, bytes, units, sc, f, cc, st); };
   const bool one = f.RE <= 32;
-  if (sc.num_colors == 3 && sc.num_sensors <= 4 && all16 && sc.combo && sc.osum) {  // staged windows
+  if (sc.num_colors == 3 && sc.num_sensors <= 4 && all16 && sc.sprod && sc.osum) {  // staged windows
     // the extraction's serial half in its own pass
     e = one ? go(fused_forward_win_kernel<1>) : go(fused_forward_win_kernel<8>);
     return e != cudaSuccess ? e : launch_extract_pass(sc, cc, f.quad, f.RE, st);

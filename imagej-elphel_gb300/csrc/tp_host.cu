@@ -46,7 +46,9 @@ struct tp_handle {
   CorrDev *d_corr_cfg = nullptr;
   float *d_tex = nullptr, *d_tex_aux = nullptr;
   float *d_combo = nullptr;  // [tiles][RE] combined strip rows of the last forward (adjoint input)
-  float *d_osum = nullptr;   // [tiles][32][8] ortho profile products handed to the extraction pass
+  float *d_sprod = nullptr;  // [tasks][RE] strip products handed to the extraction pass
+  size_t sprod_cap = 0;      // its floats
+  float *d_osum = nullptr;   // [tasks][32][8] ortho profile products handed to the extraction pass
   // Once the adjoint is in use (adj_record) the forward keeps what it needs: per-pair strip
   // samples [tiles][pairs][RE] and the plan's FP64 port derivatives
   float *d_strips = nullptr;
@@ -236,6 +238,7 @@ static SceneDev scene_of(tp_handle *h) {
   sc.clt_lpf_mask = h->lpf_on ? h->clt_lpf_mask : 0;
   sc.corr_cfg = h->d_corr_cfg;
   sc.combo = h->d_combo;
+  sc.sprod = h->d_sprod;
   sc.osum = h->d_osum;
   sc.strips = (h->adj_record && h->d_strips && strips_need(h) <= h->strips_cap) ? h->d_strips : nullptr;
   sc.tex = h->d_tex;
@@ -520,7 +523,7 @@ tp_status tp_destroy(tp_handle *h) {
                   h->d_tex, h->d_tex_aux, h->d_sens, h->d_dval, h->d_jac_e, h->d_jac_d, h->d_grad_d,
                   h->d_partial, h->d_grad_e, h->d_dldd, h->d_combo, h->d_psf_stage, h->d_rig_corr, h->d_strips, h->d_lma, h->d_mismatch,
                   h->d_pairmax,
-                  h->d_rig_rec, h->d_rig_tmp, h->d_osum};
+                  h->d_rig_rec, h->d_rig_tmp, h->d_sprod, h->d_osum};
   for (void *b : bufs) dfree(h, b);
   if (h->ev_stage) {
     cudaEventSynchronize(h->ev_stage);
@@ -1049,6 +1052,17 @@ tp_status tp_set_corr(tp_handle *h, const tp_corr_params *p, const tp_pair *pair
   if (!h->d_combo && dalloc(h, &h->d_combo, (size_t)h->ntiles * TP_MAX_STRIP * 15) != cudaSuccess) {
     cudaGetLastError();
     return fail(h, TP_ERR_NOMEM, "tp_set_corr: combined strip buffer");
+  }
+  const size_t sprod_need = (size_t)h->ntiles * (cd.strip_rows < cd.wndy_size ? cd.strip_rows : cd.wndy_size) * 15;
+  if (sprod_need > h->sprod_cap) {
+    dfree(h, h->d_sprod);
+    h->d_sprod = nullptr;
+    h->sprod_cap = 0;
+    if (dalloc(h, &h->d_sprod, sprod_need) != cudaSuccess) {
+      cudaGetLastError();
+      return fail(h, TP_ERR_NOMEM, "tp_set_corr: strip product buffer");
+    }
+    h->sprod_cap = sprod_need;
   }
   if (!h->d_osum && dalloc(h, &h->d_osum, (size_t)h->ntiles * 256) != cudaSuccess) {
     cudaGetLastError();

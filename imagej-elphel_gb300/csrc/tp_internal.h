@@ -131,8 +131,10 @@ struct SceneDev {
   const float *lpf_rbg;      // [C][64] or null
   int clt_lpf_mask;          // colours whose stored CLT is multiplied by lpf_rbg (the reference GPU's lpf_mask)
   const CorrDev *corr_cfg;
-  float *combo;              // [tiles][RE] combined strip rows the extraction reads, or null
-  float *osum;               // [tiles][32][8] per-lane ortho profile products for the separate extraction pass, or null
+  float *combo;              // [tiles][RE] combined strip rows (adjoint input), or null
+  // products of a forward with a separate extraction pass, by task: a task list may name a tile twice
+  float *sprod;              // [tasks][RE] strip products, or null
+  float *osum;               // [tasks][32][8] per-lane ortho profile products, or null
   float *strips;             // [tiles][pairs][RE] per-pair strip samples (adjoint input), or null
   float *tex;                // [tiles][rows][256] texture tiles (R, B, G, alpha[, 4 weights, 4 rms])
   float *tex_aux;            // [tiles][16] max_diff[4], ports_rgb[12] or null
@@ -184,7 +186,7 @@ cudaError_t launch_quad_batch(const SceneDev *scenes_host, const SceneDev *scene
 cudaError_t upload_many_constants();
 bool many_forward_ok(const SceneDev &sc);
 cudaError_t launch_many_forward(const SceneDev &sc, const CorrConst &cc, cudaStream_t st);
-// phase C of a forward that left its strip and ortho profile products in sc.combo and sc.osum
+// phase C of a forward that left its strip and ortho profile products in sc.sprod and sc.osum
 cudaError_t launch_extract_pass(const SceneDev &sc, const CorrConst &cc, int quad, int RE, cudaStream_t st);
 // GPU_DTT24_DRV counterpart (tp_fused.cu): 2D DTT of one mode on every 8x8 block
 cudaError_t launch_dtt8x8(float *dst, const float *src, int stride, int width, int height, int mode,

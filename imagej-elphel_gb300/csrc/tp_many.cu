@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(32 * MANY_NW, MANY_CTAS) many_kernel(const __g
     if (warp == 0 && lane < RE) {
       float v = part[lane];
       for (int w2 = 1; w2 < MANY_NW; w2++) v += part[w2 * 32 + lane];
-      sc.combo[tile * RE + lane] = v;
+      sc.sprod[(size_t)task * RE + lane] = v;
     }
   }
   if (lane == 0) bulk_done();
@@ -194,7 +194,7 @@ bool many_forward_ok(const SceneDev &sc) {
   const int RE = (sc.strip_rows < sc.wndy_size ? sc.strip_rows : sc.wndy_size) * 15;
   for (int i = 1; i < sc.num_sensors; i++)
     if (sc.img_dtype[i] != sc.img_dtype[0]) return false;
-  return sc.num_colors == 1 && sc.num_pairs > 8 && sc.all_general && RE <= 32 && sc.combo;
+  return sc.num_colors == 1 && sc.num_pairs > 8 && sc.all_general && RE <= 32 && sc.sprod;
 }
 
 cudaError_t launch_many_forward(const SceneDev &sc, const CorrConst &cc, cudaStream_t st) {

@@ -77,14 +77,14 @@ __device__ __forceinline__ void quad_clt(const SceneDev &sc, int task, SubtilePl
 
 // the products the extraction pass starts from
 template <int NT>
-__device__ __forceinline__ void store_products(const SceneDev &sc, size_t tile, int RE, int lane, const float cmb[8],
+__device__ __forceinline__ void store_products(const SceneDev &sc, size_t task, int RE, int lane, const float cmb[8],
                                                const float oprod[8]) {
 #pragma unroll
   for (int t = 0; t < NT; t++) {
     const int e = lane + 32 * t;
-    if (e < RE) sc.combo[tile * RE + e] = cmb[t];
+    if (e < RE) sc.sprod[task * RE + e] = cmb[t];
   }
-  float4 *ob = (float4 *)(sc.osum + (tile * 32 + lane) * 8);
+  float4 *ob = (float4 *)(sc.osum + (task * 32 + lane) * 8);
   ob[0] = make_float4(oprod[0], oprod[1], oprod[2], oprod[3]);
   ob[1] = make_float4(oprod[4], oprod[5], oprod[6], oprod[7]);
 }
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(128, 4) quad_kernel(const __grid_constant__ Sc
     if (next < sc.num_tasks) quad_stage<U16>(sc, p, 0, ws, q, r);  // the next tile's first windows
     float cmb[8], oprod[8];
     quad_strips<NT>(sc, cfg, surf, cur, RE, strip_code, lane, cmb, oprod);
-    store_products<NT>(sc, cur, RE, lane, cmb, oprod);
+    store_products<NT>(sc, task, RE, lane, cmb, oprod);
     if (C > 1) {  // the next tile's windows and CLT go over the surfaces
       if (lane == 0) bulk_read_done();
       __syncwarp();
@@ -219,20 +219,19 @@ __global__ void __launch_bounds__(96, 8) quad3_kernel(const __grid_constant__ Sc
   const int rr = sc.bayer_red_row, rc = sc.bayer_red_col;
   // the couple's sensors: 0-1 and 2-3, 0-2 and 1-3, 0-3 and 2-1
   const int f1 = warp == 1 ? 1 : 2, g0 = warp + 1, g1 = warp == 2 ? 1 : 3;
-  // the strip products of a tile: the values are 1 for pairs that are not combined
-  auto products = [&](size_t tile) {
+  // the strip products of a task: the values are 1 for pairs that are not combined
+  auto products = [&](size_t t) {
     if (lane < RE) {
       float v = sm[q3_strip(0, lane)];
 #pragma unroll
       for (int p = 1; p < 6; p++) v *= sm[q3_strip(p, lane)];
-      sc.combo[tile * RE + lane] = v;
+      sc.sprod[t * RE + lane] = v;
     }
   };
   int task = blockIdx.x;
   if (task >= sc.num_tasks) return;
   SubtilePlan p = quad_plan(sc, 3, task, q, warp);
   size_t tile = tile_of(sc, task), prev = 0;
-  bool have_prev = false;
   stage_window<true>(sc, sc.images[q], p.tlx, p.tly, ws + q * Stage<true>::WIN, r);
   cp_async_commit();
 #pragma unroll 1
@@ -260,9 +259,8 @@ __global__ void __launch_bounds__(96, 8) quad3_kernel(const __grid_constant__ Sc
       *(float4 *)(sdst + m * QP_QUAD) = make_float4(o[m][0], o[m][1], o[m][2], o[m][3]);
       *(float4 *)(sdst + m * QP_QUAD + 4) = make_float4(o[m][4], o[m][5], o[m][6], o[m][7]);
     }
-    if (warp == 2 && have_prev) products(prev);
+    if (warp == 2 && task >= (int)gridDim.x) products(task - gridDim.x);  // the last task's
     prev = tile;
-    have_prev = true;
     const int next = task + gridDim.x;
     const bool more = next < sc.num_tasks;
     if (more) {
@@ -298,7 +296,7 @@ __global__ void __launch_bounds__(96, 8) quad3_kernel(const __grid_constant__ Sc
           lo += stride;
           hi -= stride;
         }
-        *(float4 *)(sc.osum + (prev * 32 + warp * 16 + j) * 8 + half * 4) = make_float4(pr[0], pr[1], pr[2], pr[3]);
+        *(float4 *)(sc.osum + ((size_t)task * 32 + warp * 16 + j) * 8 + half * 4) = make_float4(pr[0], pr[1], pr[2], pr[3]);
       }
     }
 #pragma unroll
@@ -320,7 +318,7 @@ __global__ void __launch_bounds__(96, 8) quad3_kernel(const __grid_constant__ Sc
     task = next;
   }
   __syncthreads();
-  if (warp == 2) products(prev);
+  if (warp == 2) products(task);
   if (lane == 0) bulk_done();
 }
 
@@ -376,7 +374,7 @@ __global__ void __launch_bounds__(128, 4)
       if (staged) quad_stage<U16>(sc, p, 0, ws, q, r);
       float cmb[8], oprod[8];
       quad_strips<NT>(sc, cfg, surf, tile, RE, &sc.corr_cfg->strip_code[0][0][0], lane, cmb, oprod);
-      store_products<NT>(sc, tile, RE, lane, cmb, oprod);
+      store_products<NT>(sc, task, RE, lane, cmb, oprod);
     }
   }
   cp_async_wait_all();
@@ -384,8 +382,9 @@ __global__ void __launch_bounds__(128, 4)
 }
 
 // Phase C for the tiles of a fused forward that left it out: warp per task, from the strip
-// products (in sc.combo, replaced by the combined strip) and the ortho profile products (sc.osum)
-// the forward wrote.  Phase C is short chains of dependent shuffles, divides and powers; the
+// products (sc.sprod) and the ortho profile products (sc.osum) the forward wrote.  Both lie by task and the
+// combined strip goes to another buffer (sc.combo), so a tile that the task list names twice is finished twice
+// from unchanged products.  Phase C is short chains of dependent shuffles, divides and powers; the
 // fused kernel's 16 warps per SM cannot hide their latency, while this kernel's few registers
 // and no CLT buffer let 64 warps share an SM.
 template <int NT>
@@ -396,10 +395,10 @@ __device__ __forceinline__ void extract_task(const SceneDev &sc, const CorrConst
 #pragma unroll
   for (int t = 0; t < NT; t++) {
     const int e = lane + 32 * t;
-    cmb[t] = (e < RE) ? sc.combo[tile * RE + e] : 0.f;
+    cmb[t] = (e < RE) ? sc.sprod[(size_t)task * RE + e] : 0.f;
   }
   if (quad) {  // other layouts have no ortho profiles
-    const float4 *ob = (const float4 *)(sc.osum + (tile * 32 + lane) * 8);
+    const float4 *ob = (const float4 *)(sc.osum + ((size_t)task * 32 + lane) * 8);
     const float4 o0 = ob[0], o1 = ob[1];
     oprod[0] = o0.x; oprod[1] = o0.y; oprod[2] = o0.z; oprod[3] = o0.w;
     oprod[4] = o1.x; oprod[5] = o1.y; oprod[6] = o1.z; oprod[7] = o1.w;
@@ -448,7 +447,7 @@ static bool one_type(const SceneDev &sc) {
 }
 
 // a standard quad with images of one type and room for the products between the two passes
-bool quad_forward_ok(const SceneDev &sc) { return sc.quad_std && sc.combo && sc.osum && one_type(sc); }
+bool quad_forward_ok(const SceneDev &sc) { return sc.quad_std && sc.sprod && sc.osum && one_type(sc); }
 
 // a batch's mono scenes, all standard quads of the same image type
 bool quad_batch_ok(const SceneDev *h, int n) {
