@@ -1811,6 +1811,8 @@ tp_status tp_rig_correlate(tp_handle *main_h, tp_handle *aux, float cm_max_norma
   CK(launch_rig(scene_of(h), scene_of(aux), cc, h->d_rig_corr, h->d_rig_rec, cm_max_normalization, no_int_x0, st),
      "tp_rig_correlate");
   h->rig_lma_done = 0;
+  // the kernel reads the auxiliary camera's CLT and tile map: its setters wait for it as the main camera's do
+  if (aux != h && mark_work(aux, st) != TP_OK) return fail(h, TP_ERR_CUDA, aux->err);
   return mark_work(h, st);
 }
 
