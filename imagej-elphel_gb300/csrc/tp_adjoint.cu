@@ -33,6 +33,7 @@
 // gradient with one warp's shared-memory atomics); finally the warps split the
 // sensors for the forward-mode shift derivatives.
 #include "tp_adjoint.cuh"
+#include "tp_pairs.cuh"
 #include "tp_launch.h"
 
 __global__ void __launch_bounds__(32 * AD_NW, 4) adjoint_kernel(const __grid_constant__ SceneDev sc,
@@ -391,6 +392,23 @@ __global__ void __launch_bounds__(256) adjoint_final_kernel(const float *partial
   if (t == 0) grad_e[i] = s[0];
 }
 
+// The strip samples of a forward that did not record them, from its stored surfaces (the recorded values' bits: the
+// forward's own functions on the same surfaces): a warp per (task, pair), strips of at most 32 entries.  With them
+// the per-tile kernel of a scene does not depend on what the handle ran before.
+__global__ void __launch_bounds__(128) sample_strips_kernel(const __grid_constant__ SceneDev sc, int RE) {
+  const int lane = threadIdx.x & 31, P = sc.num_pairs;
+  const int i = blockIdx.x * 4 + (threadIdx.x >> 5), task = i / P, pi = i - task * P;
+  if (task >= sc.num_tasks || lane >= RE) return;
+  const CorrDev &cd = *sc.corr_cfg;
+  const int kind = cd.pairs[pi].kind;
+  if (!cd.pairs[pi].in_combo) return;
+  const int txy = sc.task_txy[task];
+  const size_t at = ((size_t)(txy >> 16) * sc.tilesX + (txy & 0xffff)) * P + pi;
+  const float *c = sc.corr + at * TP_CORR;
+  sc.strips[at * RE + lane] = kind == 4 ? tap_strip(c, *((const float4 *)cd.gen_tap[pi] + lane), cd.gen_cell[pi][lane], lane >= 15)
+                                        : strip_of(c, quad_code(&cd.strip_code[0][0][0], kind, lane), lane);
+}
+
 cudaError_t upload_adjoint_constants() {
   cudaError_t e = upload_dtt_constants();
   if (e != cudaSuccess) return e;
@@ -415,10 +433,14 @@ cudaError_t launch_adjoint(const SceneDev &sc, const CorrConst &cc, int recomput
   as.use_strips = (use_strips && sc.strips) ? 1 : 0;
   const int bytes = adjoint_smem_bytes(as.S, as.C);
   cudaError_t e;
-  if (as.use_strips && adjoint_many_ok(sc, recompute)) {
-    e = launch_adjoint_many(sc, cc, sens, dval, st);
-  } else if (as.use_strips && adjoint_quad_ok(sc, recompute)) {
-    e = launch_adjoint_quad(sc, cc, sens, dval, st);
+  const bool many = sc.strips && adjoint_many_ok(sc, recompute), quad = sc.strips && adjoint_quad_ok(sc, recompute);
+  if (many || quad) {
+    if (!as.use_strips) {
+      sample_strips_kernel<<<(sc.num_tasks * sc.num_pairs + 3) / 4, 128, 0, st>>>(sc, as.RE);
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+    }
+    e = many ? launch_adjoint_many(sc, cc, sens, dval, st) : launch_adjoint_quad(sc, cc, sens, dval, st);
   } else {
     int res = 0;
     e = kernel_residency((const void *)adjoint_kernel, 32 * AD_NW, bytes, &res);

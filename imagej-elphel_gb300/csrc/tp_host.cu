@@ -1910,6 +1910,7 @@ tp_status tp_backward(tp_handle *h, const float *dl_ddisp, float *dl_dextr, floa
   const int use_strips = h->strips_valid && sc.strips;
   tp_status rs = enable_strip_recording(h);  // later forwards keep their strip samples and derivatives
   if (rs != TP_OK) return rs;
+  sc.strips = h->d_strips;
   if (!h->deriv_valid) CK(launch_plan(sc, st), "tp_backward plan");
   h->deriv_valid = 1;
   if (dl_ddisp) CK(cudaMemcpyAsync(h->d_dldd, dl_ddisp, nt * sizeof(float), cudaMemcpyHostToDevice, st), "tp_backward");

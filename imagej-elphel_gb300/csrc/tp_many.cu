@@ -38,17 +38,6 @@ __device__ __forceinline__ void store_surface(float *g, const float *s, int mis,
   if (lane < 4 ? i < head : (lane < 8 && i < 225)) g[i] = s[i];
 }
 
-// one strip entry from its taps (strip_sample, both sides below the first row)
-__device__ __forceinline__ float tap_sample(const float *c, float dx, float dy) {
-  const float w00 = (1.0f - dx) * (1.0f - dy), w10 = dx * (1.0f - dy), w01 = (1.0f - dx) * dy, w11 = dx * dy;
-  return fmaf(w11, c[16], fmaf(w01, c[15], fmaf(w00, c[0], w10 * c[1])));
-}
-__device__ __forceinline__ float tap_strip(const float *c, float4 tap, int cells, bool both) {
-  const float d = tap_sample(c + (cells & 255), tap.x, tap.y), d2 = tap_sample(c + ((cells >> 8) & 255), tap.z, tap.w);
-  const bool out = (cells & 0x10000) || (both && (cells & 0x20000));
-  return out ? CUDART_NAN_F : (both ? 0.5f * d + 0.5f * d2 : d);
-}
-
 // the normalised, filtered spectra of two pairs into b (interleaved [4][8][9]); the pairs are numbered by their first
 // sensor, which two that lie four apart mostly share
 __device__ __forceinline__ void couple_spectra(const CorrConst &cfg, const PairDev &pa, const PairDev &pb, float2 l0,

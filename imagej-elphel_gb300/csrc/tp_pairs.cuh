@@ -319,6 +319,17 @@ __device__ __forceinline__ short2 quad_code(const short *strip_code, int kind, i
   return *(const short2 *)&strip_code[(kind * TP_MAX_STRIP * 15 + e) * 2];
 }
 
+// one strip entry of a general pair from its taps (CorrDev::gen_tap; strip_sample, both sides below the first row)
+__device__ __forceinline__ float tap_sample(const float *c, float dx, float dy) {
+  const float w00 = (1.0f - dx) * (1.0f - dy), w10 = dx * (1.0f - dy), w01 = (1.0f - dx) * dy, w11 = dx * dy;
+  return fmaf(w11, c[16], fmaf(w01, c[15], fmaf(w00, c[0], w10 * c[1])));
+}
+__device__ __forceinline__ float tap_strip(const float *c, float4 tap, int cells, bool both) {
+  const float d = tap_sample(c + (cells & 255), tap.x, tap.y), d2 = tap_sample(c + ((cells >> 8) & 255), tap.z, tap.w);
+  const bool out = (cells & 0x10000) || (both && (cells & 0x20000));
+  return out ? CUDART_NAN_F : (both ? 0.5f * d + 0.5f * d2 : d);
+}
+
 // First half of a standard quad's pair phase: the six surfaces to ws + QP_SURF and, asynchronously, to
 // HBM; returns where they are.  The spectra's space (up to QP_SURF) is then free; the caller waits
 // (bulk_read_done by lane 0, then __syncwarp) before it writes the surfaces' space again.

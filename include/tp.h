@@ -451,7 +451,9 @@ tp_status tp_batch_synchronize(tp_batch *b);
  * dl_dextr [num_sensors][4] and dl_dtile_disp [tilesY*tilesX] are host
  * outputs (either may be NULL).  From the first tp_backward (or
  * tp_set_adjoint_mode) on, tp_process also records every pair's strip samples
- * ([tiles][pairs][strip entries] floats on the device) for the adjoint to read. */
+ * ([tiles][pairs][strip entries] floats on the device) for the adjoint to read;
+ * a forward that did not is sampled again from its surfaces, with the same results
+ * (bit for bit; the recomputed CLT of tp_set_adjoint_mode sums in another order). */
 tp_status tp_backward(tp_handle *h, const float *dl_ddisp, float *dl_dextr, float *dl_dtile_disp, void *stream);
 /* 1: the adjoint recomputes each tile's CLT from the images instead of reading
  * the stored CLT back (for when the CLT buffer is not kept; a Bayer colour as the
