@@ -102,7 +102,10 @@ __global__ void __launch_bounds__(32 * MANY_NW, MANY_CTAS) many_kernel(const __g
   const float2 l0 = dup2(0.25f * cfg.lpf[lane]), l1 = dup2(0.25f * cfg.lpf[lane + 32]);
   const int s = min(warp * 4 + q, S - 1);  // the sensor whose window and CLT this lane works on
   const bool act = warp * 4 + q < S, has_group = warp < groups;
-  for (int task = blockIdx.x; task < sc.num_tasks; task += gridDim.x) {
+  // where the task's products go, carried along: worked out at the store it cost 4 us in 16x640x512 (422.7 and
+  // 419.6 us a pass; by tile as the surfaces 419.0)
+  float *out = sc.sprod + (size_t)blockIdx.x * RE + lane;
+  for (int task = blockIdx.x; task < sc.num_tasks; task += gridDim.x, out += (size_t)gridDim.x * RE) {
     const int txy = sc.task_txy[task];
     const size_t tile = (size_t)(txy >> 16) * sc.tilesX + (txy & 0xffff);
     if (has_group) {
@@ -170,7 +173,7 @@ __global__ void __launch_bounds__(32 * MANY_NW, MANY_CTAS) many_kernel(const __g
     if (warp == 0 && lane < RE) {
       float v = part[lane];
       for (int w2 = 1; w2 < MANY_NW; w2++) v += part[w2 * 32 + lane];
-      sc.sprod[(size_t)task * RE + lane] = v;
+      *out = v;
     }
   }
   if (lane == 0) bulk_done();
