@@ -5,7 +5,7 @@
 // takes two pairs at once, one in each half of the packed FP32 registers, so a round holds up to eight
 // pairs on distinct sensors (16 sensors: 15 rounds of 8); the strip taps come from the forward's table;
 // and the windows of the shift derivatives are staged (tp_forward.cuh).
-// Needs the forward's strip samples (SceneDev::strips) and a strip of at most 32 entries.
+// Needs the forward's strip samples (SceneDev::strips, recorded or sampled again) and a strip of at most 32 entries.
 // Measured on 16x640x512 (5,120 tiles, 120 pairs): 992 -> 640 us; 617 with the windows over a group's CLT once it is
 // read, which leaves room for a fifth CTA an SM (96 registers; with 128 and four CTAs 643).  What bounds it
 // now: the shared-memory pipe (about 70 %: the pairs' CLT reads and gradient updates are 96 of some 350 accesses a

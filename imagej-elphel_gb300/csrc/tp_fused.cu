@@ -594,7 +594,7 @@ __device__ __forceinline__ void dct4_two(const float2 x[8], float2 y[8]) {
 
 constexpr int IMCLT_IR = 10;      // region = IR x IR blocks of 8x8 pixels
 constexpr int IMCLT_WARPS = 5;    // the four parity phases (25, 30, 30, 36 tiles), four tiles a warp, in two rounds each
-constexpr int IMCLT_SMALL = 152;  // regions for a region on each SM
+constexpr int IMCLT_SMALL = 152;  // regions for a region on each of the chip's SMs
 
 template <int IR, int NW>
 __global__ void __launch_bounds__(32 * NW) imclt_fast_kernel(const __grid_constant__ SceneDev sc) {

@@ -1850,7 +1850,7 @@ tp_status tp_get_rig(tp_handle *h, float *corr, float *rec) {
 }
 
 // From the first adjoint on, the forward records every pair's strip samples [tiles][pairs][RE]
-// so the adjoint reads them instead of re-interpolating the correlation surfaces.
+// so the adjoint reads them instead of interpolating the correlation surfaces again.
 static tp_status enable_strip_recording(tp_handle *h) {
   const size_t need = strips_need(h);
   if (need > h->strips_cap) {

@@ -211,11 +211,11 @@ cudaError_t launch_compact_tasks_scratch(const int *tile_op, const float *dispar
 // adjoint (tp_adjoint.cu): per-tile dd/dport, Jacobian rows, loss gradient
 cudaError_t upload_adjoint_constants();
 int adjoint_smem_bytes(int S, int C);
-// its per-tile kernel for Bayer standard quads with recorded strips (tp_adjoint_quad.cu)
+// its per-tile kernel for Bayer standard quads (tp_adjoint_quad.cu); reads sc.strips
 cudaError_t upload_adjoint_quad_constants();
 bool adjoint_quad_ok(const SceneDev &sc, int recompute);
 cudaError_t launch_adjoint_quad(const SceneDev &sc, const CorrConst &cc, float *sens, float *dval, cudaStream_t st);
-// its per-tile kernel for mono scenes with many general pairs and recorded strips (tp_adjoint_many.cu)
+// its per-tile kernel for mono scenes with many general pairs (tp_adjoint_many.cu); reads sc.strips
 cudaError_t upload_adjoint_many_constants();
 bool adjoint_many_ok(const SceneDev &sc, int recompute);
 cudaError_t launch_adjoint_many(const SceneDev &sc, const CorrConst &cc, float *sens, float *dval, cudaStream_t st);

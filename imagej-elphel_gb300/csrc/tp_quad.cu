@@ -10,7 +10,8 @@
 // Measured (kernel and extraction together, general schedule -> now): 4x2592x1936 u16 Bayer with kernel
 // tables, 78,408 tiles: 0.922 -> 0.756 ms; 4x1304x984 float Bayer, 7,018 tiles: 129 -> 80 us; 16 batched
 // 4x512x384 float mono scenes, 49,152 tiles: 452 -> 316 us.  What bounds it now: latency at 16 warps
-// an SM (128 registers a thread): the issue slots and the shared-memory pipe are a little over half used.
+// an SM (128 registers a thread).  Issue slots and shared-memory pipe in use: 41 and 36 % at 3,072 mono tiles, 51
+// and 47 % at 7,018 float Bayer tiles, 51 and 59 % over the 16 batched scenes.
 //
 // Shared memory of a warp (floats): CLT [C][4 sensors][QP_CLT] first; the windows of colour item c at
 // 4 QP_CLT c (where that item's CLT goes once they are read); the pairs' spectra over the CLT
@@ -200,12 +201,14 @@ __device__ __forceinline__ void conv_shift_pairs(float o[4][8], const float *kp,
 // transposes go too.
 // 4 x 2592x1936 with kernel tables, 78,408 tiles: warp per tile 729 us, this 728, with conv_shift_pairs
 // 693 (packed, the warp per tile spills: 746); 4 x 648x488, 4,941 tiles: 52 -> 46.  The price is that each warp
-// reads the whole CLT (288 shared-memory accesses a tile instead of 96), so that pipe is at 65 % and the issue
-// slots at 65 %; float windows are too large for eight CTAs an SM (7,018 tiles: 73 us warp per tile, 75 here), so
+// reads the whole CLT (288 shared-memory accesses a tile instead of 96), so that pipe is at 69 % and the issue
+// slots at 59 % (4 x 1296x968); float windows are too large for eight CTAs an SM (7,018 tiles: 73 us warp per tile, 75 here), so
 // they stay with a warp per tile.
 constexpr int Q3_SURF = 4 * Stage<true>::WIN;       // first surface (+ 0 or 2 floats)
 constexpr int Q3_WS = Q3_SURF + 456;                // scratch of a warp
-constexpr int Q3_FLOATS = 12 * QP_CLT + 3 * Q3_WS;  // 28,896 bytes with the 1 KB a CTA costs: eight in 228 KB
+// 29,152 bytes with the 1 KB a CTA costs: eight in 228 KB, with 32 bytes left for each (static shared memory, of which
+// the kernel has none, is not in the assertion)
+constexpr int Q3_FLOATS = 12 * QP_CLT + 3 * Q3_WS;
 static_assert(Q3_SURF >= QP_BUF && 8 * (4 * Q3_FLOATS + 1024) <= 228 * 1024, "spectra over the windows, eight CTAs");
 // strip value e of pair p: [6][32] in the 4 unused floats of each of the 48 quadrants
 __device__ __forceinline__ int q3_strip(int p, int e) { return (p * 8 + (e >> 2)) * QP_QUAD + 32 + (e & 3); }

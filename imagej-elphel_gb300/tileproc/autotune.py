@@ -3,10 +3,16 @@
 Candidates (tp_set_schedule), spanning tiles per CTA x warps per tile x register
 budget:
   (1, 1), (2, 2), (4, 4)  one warp per tile, 1 / 2 / 4 tiles per CTA, up to 128
-                          registers (4 CTAs of 4 warps per SM); for u16 Bayer quads
-                          with staged image windows;
+                          registers (4 CTAs of 4 warps per SM).  A standard quad
+                          with images of one type runs its own kernel here, with 1 / 2 / 4
+                          warps per CTA; a u16 Bayer one with strips of at most two
+                          rows the same three-warp kernel under all of them, so that
+                          a pick among the three is chance;
   (1, 2), (1, 4)          one tile per CTA, its colour items and pairs split over 2 / 4
-                          warps sharing the tile's CLT, up to 128 registers;
+                          warps sharing the tile's CLT, up to 128 registers.  (1, 4) on a
+                          mono scene of one image type with more than 8 pairs, all of
+                          kind 4, and strips of at most two rows runs the many-pair
+                          kernel (two pairs per warp, 80 registers);
   (1, 3)                  one tile per CTA of 3 warps (one colour item, then two pairs
                           per warp for a quad colour scene), 80 registers for 8 CTAs
                           (24 warps) per SM.

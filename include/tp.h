@@ -209,7 +209,9 @@ tp_status tp_set_image_async(tp_handle *h, int cam, const void *image, int dtype
  * before the GPU mosaic is formed); default {1, 1, 1} for R, B, G */
 tp_status tp_set_color_scales(tp_handle *h, const float *scales);
 /* setTasks (GPUTileProcessor.java:363-371): TpTask.asFloatArray layout,
- * per task {task (int bits), tx | ty << 16 (int bits), xy[num_sensors][2]} */
+ * per task {task (int bits), tx | ty << 16 (int bits), xy[num_sensors][2]}.  A tile may occur
+ * more than once (at most tilesX * tilesY tasks in all): with the same ports in every entry its
+ * results are those of one entry, with different ones it is not defined whose they are. */
 tp_status tp_set_tasks(tp_handle *h, const float *packed_tasks, int num_tasks);
 /* setFullFrameImages(float[] target_disparities) + getTileSubcamOffsets
  * (GPUTileProcessor.java:472-527, 686-778) computed on the device in FP64:
@@ -414,7 +416,10 @@ tp_status tp_rig_lma(tp_handle *main_camera, const tp_lma_params *p, int use_pol
  * warp-per-tile, mono with more than 8 pairs: 4 warps per tile) over a queue
  * of tiles in scene order, the classes running concurrently.  Warp-per-tile
  * scenes with at least 8 waves of tiles (8 x 16 x SM count) keep their own
- * forward launch inside the same step (they have no tail to share).  Colour
+ * forward launch inside the same step (they have no tail to share), and so do
+ * mono scenes of one image type with more than 8 pairs, all of kind 4, strips of
+ * at most two rows and the default or the (1, 4) schedule from one wave of
+ * tiles on (6 x SM count).  Colour
  * scenes need sensors x colours <= 16 and at most 8 pairs.  The handles stay owned by the caller and must
  * outlive the batch; results are read through each handle's getters. */
 typedef struct tp_batch tp_batch;
