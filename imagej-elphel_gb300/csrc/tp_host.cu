@@ -46,7 +46,8 @@ struct tp_handle {
   CorrDev *d_corr_cfg = nullptr;
   float *d_tex = nullptr, *d_tex_aux = nullptr;
   float *d_combo = nullptr;  // [tiles][RE] combined strip rows of the last forward (adjoint input)
-  float *d_sprod = nullptr;  // [tasks][RE] strip products handed to the extraction pass
+  float *d_sprod = nullptr;  // [tasks][RE] strip products handed to the extraction pass, for strips of more than
+                             // half of TP_MAX_STRIP rows (others: the part of d_combo that the strips leave free)
   size_t sprod_cap = 0;      // its floats
   float *d_osum = nullptr;   // [tasks][32][8] ortho profile products handed to the extraction pass
   // Once the adjoint is in use (adj_record) the forward keeps what it needs: per-pair strip
@@ -195,6 +196,14 @@ static int is_standard_quad(const tp_handle *h) {
   return 1;
 }
 
+// the strip products handed to the extraction pass (null: no room, the forward then takes the general kernels)
+static float *strip_products(const tp_handle *h) {
+  const int rows = h->corr_host.strip_rows < h->corr_host.wndy_size ? h->corr_host.strip_rows : h->corr_host.wndy_size;
+  const size_t need = (size_t)h->ntiles * rows * 15;
+  if (2 * rows <= TP_MAX_STRIP) return h->d_combo ? h->d_combo + need : nullptr;
+  return need <= h->sprod_cap ? h->d_sprod : nullptr;
+}
+
 static SceneDev scene_of(tp_handle *h) {
   SceneDev sc;
   memset(&sc, 0, sizeof(sc));
@@ -238,7 +247,7 @@ static SceneDev scene_of(tp_handle *h) {
   sc.clt_lpf_mask = h->lpf_on ? h->clt_lpf_mask : 0;
   sc.corr_cfg = h->d_corr_cfg;
   sc.combo = h->d_combo;
-  sc.sprod = h->d_sprod;
+  sc.sprod = strip_products(h);
   sc.osum = h->d_osum;
   sc.strips = (h->adj_record && h->d_strips && strips_need(h) <= h->strips_cap) ? h->d_strips : nullptr;
   sc.tex = h->d_tex;
@@ -1053,16 +1062,14 @@ tp_status tp_set_corr(tp_handle *h, const tp_corr_params *p, const tp_pair *pair
     cudaGetLastError();
     return fail(h, TP_ERR_NOMEM, "tp_set_corr: combined strip buffer");
   }
-  const size_t sprod_need = (size_t)h->ntiles * (cd.strip_rows < cd.wndy_size ? cd.strip_rows : cd.wndy_size) * 15;
-  if (sprod_need > h->sprod_cap) {
+  const int rows = cd.strip_rows < cd.wndy_size ? cd.strip_rows : cd.wndy_size;
+  const size_t sprod_need = 2 * rows <= TP_MAX_STRIP ? 0 : (size_t)h->ntiles * rows * 15;
+  if (sprod_need > h->sprod_cap) {  // optional (strip_products)
     dfree(h, h->d_sprod);
     h->d_sprod = nullptr;
     h->sprod_cap = 0;
-    if (dalloc(h, &h->d_sprod, sprod_need) != cudaSuccess) {
-      cudaGetLastError();
-      return fail(h, TP_ERR_NOMEM, "tp_set_corr: strip product buffer");
-    }
-    h->sprod_cap = sprod_need;
+    if (dalloc(h, &h->d_sprod, sprod_need) == cudaSuccess) h->sprod_cap = sprod_need;
+    else cudaGetLastError();
   }
   if (!h->d_osum && dalloc(h, &h->d_osum, (size_t)h->ntiles * 256) != cudaSuccess) {
     cudaGetLastError();
